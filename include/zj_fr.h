@@ -238,7 +238,7 @@ zj_status zj_rhs_noalloc(zj_solver* s, const double* U_dev, double* R_dev);
  * Replace MeshPartitioner::partition (src/mesh/partitioner.cpp:10-93, METIS
  * k-way on the element dual graph) and MPICommunicator::exchangeHalo
  * (src/parallel/mpi_comm.cpp:68-171).  A partitioned mesh runs as one handle
- * per part; the parts couple only through the traces and gradient traces at
+ * per part; the parts couple only through the traces and viscous shares at
  * the faces the partition cuts, which cross after every launch that writes
  * them: the sender gathers its side's trace rows, the receiver copies them
  * into its own memory (a peer copy between devices) and scatters them into
@@ -283,8 +283,8 @@ zj_status zj_parts_residual_norm(zj_solver* const* parts, int n, double* out);
 /* One process per GPU (the caller's MPI or NCCL moves the rows; the
  * reference's MPICommunicator::exchangeHalo, mpi_comm.cpp:68-171): nsteps
  * SSP-RK3 steps of the part s alone, on its stream.  At each exchange (the
- * state traces before the first step, then per stage the gradient traces
- * after the gradient launch (Navier-Stokes) and the new traces after the
+ * state traces before the first step, then per stage the faces' viscous
+ * shares after the gradient launch (Navier-Stokes) and the new traces after the
  * stage launch) the part's cut-face rows are gathered into send_dev, in the
  * halo plan's order (zj_halo_plan: rows [nbr_off[i], nbr_off[i+1]) for
  * neighbour nbr[i]; row_bytes bytes each), and exchange(user, kind,

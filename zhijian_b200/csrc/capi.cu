@@ -7,7 +7,7 @@
 //                                  zj_rhs (+ boundary ghost rows)
 //   metrics [E][n_sp][4] Jinv, [E][n_sp] J, per-element edge records, bc
 //   scratch state + residual for the host-buffer entry points, reductions
-// Traces, gradient traces, metrics, normals, operators and bc data exist in
+// Traces, viscous shares, metrics, normals, operators and bc data exist in
 // the arithmetic type of the handle: FP64, or FP32 for the mixed-precision
 // form (whose state and reductions stay FP64).
 // An SSP-RK3 step is three fused stage launches; the first step after a state
@@ -41,7 +41,7 @@ struct zj_solver {
     size_t state_n = 0, trace_n = 0;
     double* dU[3] = {nullptr, nullptr, nullptr};
     double* dT[3] = {nullptr, nullptr, nullptr};
-    double* dTQ = nullptr;      // gradient traces (Navier-Stokes)
+    double* dTQ = nullptr;      // viscous shares of the faces, or gradient traces (Navier-Stokes)
     double* dUs = nullptr;      // scratch state (host-buffer residual)
     double* dRs = nullptr;      // scratch residual
     double* dJinv = nullptr;
@@ -57,7 +57,7 @@ struct zj_solver {
     int* dFlag = nullptr;
     EdgeRec* dEdges = nullptr;
     double4* dNrm = nullptr;
-    // mixed-precision form: FP32 traces, gradient traces and geometry
+    // mixed-precision form: FP32 traces, viscous shares and geometry
     bool mixed = false;
     int nrm_pp = 0;             // curved elements in physics mode: normals per flux point
     float* fT[3] = {nullptr, nullptr, nullptr};
@@ -241,13 +241,13 @@ template <typename T> StageArgsT<T> base_args(const zj_solver* s);
 template <> StageArgsT<double> base_args<double>(const zj_solver* s) {
     StageArgsT<double> a{};
     a.Jinv = s->dJinv; a.J = s->dJ; a.enrm = s->dNrm; a.bc = s->dBC; a.ops = s->dOps;
-    a.TQ = s->dTQ; a.TQout = s->dTQ; a.nrm_pp = s->nrm_pp;
+    a.FV = s->dTQ; a.FVout = s->dTQ; a.nrm_pp = s->nrm_pp;
     return a;
 }
 template <> StageArgsT<float> base_args<float>(const zj_solver* s) {
     StageArgsT<float> a{};
     a.Jinv = s->fJinv; a.J = s->fJ; a.enrm = s->fNrm; a.bc = s->fBC; a.ops = s->fOps;
-    a.TQ = s->fTQ; a.TQout = s->fTQ; a.nrm_pp = s->nrm_pp;
+    a.FV = s->fTQ; a.FVout = s->fTQ; a.nrm_pp = s->nrm_pp;
     return a;
 }
 
@@ -292,7 +292,7 @@ cudaError_t launch_stage(const zj_solver* s, const StageArgsT<T>& a) {
         }
         return launch_ns_stage(s->P, s->prm.riemann, a, s->stream);
     }
-    // quads and triangles: every gradient trace before any stage (a face's
+    // quads and triangles: every viscous share before any stage (a face's
     // neighbour may be of the other kind); the triangles' CTAs write their
     // partial sums after the quads'
     StageArgsT<T> q = a, t = a;
@@ -448,16 +448,16 @@ zj_status step_impl(zj_solver* s, int nsteps, double dt) {
     return ZJ_OK;
 }
 
-// Residual of U_dev into R_dev with the given trace / gradient-trace /
+// Residual of U_dev into R_dev with the given trace / viscous-share /
 // partial-sum scratch.
 template <typename T>
-zj_status rhs_impl(zj_solver* s, const double* U_dev, double* R_dev, T* traces, T* grad_traces,
+zj_status rhs_impl(zj_solver* s, const double* U_dev, double* R_dev, T* traces, T* face_shares,
                    double* partials) {
     ZJ_CK(s, launch_trace_any(s, U_dev, traces), "trace launch");
     StageArgsT<T> a = stage_args<T>(s);
     a.U = U_dev; a.U0 = U_dev; a.Uout = nullptr; a.Tin = traces; a.Tout = nullptr;
     a.R = R_dev; a.partials = partials; a.stage = 0;
-    if (grad_traces) { a.TQ = grad_traces; a.TQout = grad_traces; }
+    if (face_shares) { a.FV = face_shares; a.FVout = face_shares; }
     ZJ_CK(s, launch_stage(s, a), "residual launch");
     return ZJ_OK;
 }
@@ -989,8 +989,8 @@ zj_status zj_rhs_noalloc(zj_solver* s, const double* U_dev, double* R_dev) {
     double* scratch = nullptr;
     ZJ_CK(s, noalloc_scratch(&scratch), "static scratch address");
     // Every scratch value is written before it is read (all traces by the
-    // trace launch, the gradient traces by the gradient launch, one partial
-    // per CTA), so nothing needs clearing.  The gradient traces (read and
+    // trace launch, the viscous shares by the gradient launch, one partial
+    // per CTA), so nothing needs clearing.  The shares (read and
     // written as 32-byte rows) come first, at the array's 256-byte aligned
     // start; the traces follow at 2 trace_n values (a multiple of 32 bytes,
     // trace_n being a multiple of 4), the partials after them at a multiple of
@@ -1070,7 +1070,7 @@ zj_status jvp_core(zj_solver* s, const double* U, const double* V, double dRe, d
     set_viscous_constants(a);
     a.U = U; a.U0 = U; a.dU = V; a.Tout = s->xT;
     ZJ_CK(s, launch_phys_traces(s->P, a, s->stream), "jvp trace launch");
-    a.Tin = s->xT; a.TQ = s->xTQ; a.TQout = s->xTQ;
+    a.Tin = s->xT; a.FV = s->xTQ; a.FVout = s->xTQ;
     a.R = R ? R : s->aR; a.dR = JV; a.partials = s->xPart; a.stage = 0;
     if (is_ns(s)) {
         ZJ_CK(s, launch_ns_grad(s->P, a, s->stream), "jvp gradient launch");
@@ -1102,7 +1102,7 @@ zj_status vjp_core(zj_solver* s, const double* U, const double* L, double* W, do
         T = s->dT[2];
         if (is_ns(s)) {
             StageArgs a = stage_args<double>(s);
-            a.U = U; a.Tin = T; a.TQout = s->dTQ;
+            a.U = U; a.Tin = T; a.FVout = nullptr; a.GQ = s->dTQ;
             ZJ_CK(s, launch_ns_grad(s->P, a, s->stream), "vjp gradient launch");
             TQ = s->dTQ;
         }
@@ -1147,25 +1147,26 @@ struct StageTraces {
 // state into Xout (may be X).  Without keep, uses the stepper's trace
 // buffers; with keep, writes every stage input's traces and gradient traces
 // into keep's buffers (the third stage's gradient traces even when Xout is
-// NULL).
+// NULL); the faces' viscous shares stay in the handle's buffer.
 zj_status rk3_stages(zj_solver* s, const double* X, double* S1, double* S2, double* Xout,
                      const StageTraces* keep = nullptr) {
     double* T[3] = {s->dT[0], s->dT[1], s->dT[0]};
-    double* TQ[3] = {s->dTQ, s->dTQ, s->dTQ};
+    double* GQ[3] = {nullptr, nullptr, nullptr};
     if (keep)
-        for (int k = 0; k < 3; ++k) { T[k] = keep->T[k]; TQ[k] = keep->TQ[k]; }
+        for (int k = 0; k < 3; ++k) { T[k] = keep->T[k]; GQ[k] = keep->TQ[k]; }
     ZJ_CK(s, launch_trace_any(s, X, T[0]), "trace launch");
     StageArgs a = stage_args<double>(s);
     a.partials = s->dPartR;
-    a.U = X; a.U0 = X; a.Uout = S1; a.Tin = T[0]; a.Tout = T[1]; a.TQ = a.TQout = TQ[0]; a.stage = 1;
+    a.U = X; a.U0 = X; a.Uout = S1; a.Tin = T[0]; a.Tout = T[1]; a.GQ = GQ[0]; a.stage = 1;
     ZJ_CK(s, launch_stage(s, a), "stage 1 launch");
-    a.U = S1; a.Uout = S2; a.Tin = T[1]; a.Tout = T[2]; a.TQ = a.TQout = TQ[1]; a.stage = 2;
+    a.U = S1; a.Uout = S2; a.Tin = T[1]; a.Tout = T[2]; a.GQ = GQ[1]; a.stage = 2;
     ZJ_CK(s, launch_stage(s, a), "stage 2 launch");
-    a.U = S2; a.Tin = T[2]; a.TQ = a.TQout = TQ[2];
+    a.U = S2; a.Tin = T[2]; a.GQ = GQ[2];
     if (Xout) {
         a.Uout = Xout; a.Tout = s->dT[1]; a.stage = 3;
         ZJ_CK(s, launch_stage(s, a), "stage 3 launch");
     } else if (keep && is_ns(s)) {
+        a.FVout = nullptr;
         ZJ_CK(s, launch_ns_grad(s->P, a, s->stream), "gradient launch");
     }
     s->traces_valid = false;   // the stepper's traces now hold this step's
@@ -1541,7 +1542,7 @@ zj_status zj_solver_create_from_gmsh(const char* msh_path, const zj_params* para
 
 // ------------------------------------------------------- mesh partitions --
 // A partitioned mesh runs as one handle per part (zj_solver_create_part);
-// the parts couple only through the traces and gradient traces at the faces
+// the parts couple only through the traces and viscous shares at the faces
 // their partition cuts.  Each part's interface faces read the other side's
 // trace rows from ghost rows, which an exchange fills after every launch that
 // writes traces: the sender gathers its side's rows into a send buffer in the
@@ -1594,7 +1595,7 @@ zj_status parts_check(zj_solver* const* parts, int n, std::vector<zj_solver*>& b
 }
 
 // Rows of width w of every part's buffer bufs[rank] (trace rows: n1*4 values,
-// gradient trace rows: n1*8) across the cuts.
+// viscous-share rows the same) across the cuts.
 template <typename T>
 zj_status parts_exchange(const std::vector<zj_solver*>& P, const std::vector<T*>& bufs, int w) {
     const int threads = 256;
@@ -1652,7 +1653,7 @@ template <> double* grad_buf<double>(const zj_solver* s) { return s->dTQ; }
 template <> float* grad_buf<float>(const zj_solver* s) { return s->fTQ; }
 
 // The stage launch of a part (physics mode, quadrilaterals): the
-// Navier-Stokes stage after its gradient traces crossed, else the inviscid
+// Navier-Stokes stage after its viscous shares crossed, else the inviscid
 // stage.
 template <typename T>
 cudaError_t launch_part_stage(zj_solver* s, const StageArgsT<T>& a) {
@@ -1668,7 +1669,7 @@ cudaError_t launch_part_stage(zj_solver* s, const StageArgsT<T>& a) {
 }
 
 // One residual (stage 0) or SSP-RK3 stage of every part: for Navier-Stokes
-// the gradient launches, their gradient traces across the cuts, then the
+// the gradient launches, their viscous shares across the cuts, then the
 // stage launches; a stage's new traces cross after it.
 template <typename T>
 zj_status parts_stage(const std::vector<zj_solver*>& P, const std::vector<StageArgsT<T>>& A) {
@@ -1680,7 +1681,7 @@ zj_status parts_stage(const std::vector<zj_solver*>& P, const std::vector<StageA
             ZJ_CK(P[i], launch_ns_grad(P[i]->P, A[i], P[i]->stream), "gradient launch");
             tq.push_back(grad_buf<T>(P[i]));
         }
-        zj_status st = parts_exchange<T>(P, tq, P[0]->n1 * 8);
+        zj_status st = parts_exchange<T>(P, tq, P[0]->n1 * 4);
         if (st != ZJ_OK) return st;
     }
     std::vector<T*> out;
@@ -1884,7 +1885,7 @@ zj_status part_step_t(zj_solver* s, int nsteps, zj_exchange_fn fn, void* user, d
             const StageArgsT<T> a = part_stage_args<T>(s, stage);
             if (is_ns(s)) {
                 ZJ_CK(s, launch_ns_grad(s->P, a, s->stream), "gradient launch");
-                if ((st = part_exchange_cb<T>(s, grad_buf<T>(s), s->n1 * 8, ZJ_XCHG_GRADIENTS, fn, user)) != ZJ_OK)
+                if ((st = part_exchange_cb<T>(s, grad_buf<T>(s), s->n1 * 4, ZJ_XCHG_GRADIENTS, fn, user)) != ZJ_OK)
                     return st;
             }
             ZJ_CK(s, launch_part_stage<T>(s, a), "stage launch");

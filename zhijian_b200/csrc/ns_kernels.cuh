@@ -5,11 +5,22 @@
 // per residual:
 //
 //  k_ns_grad_lines (float, double; k_ns_grad for dual numbers)
-//              corrected gradient Q = grad U at the solution points and its
-//              traces at the flux points (written for the neighbours);
+//              corrected gradient Q = grad U at the solution points, its
+//              traces at the flux points and, from them, this element's share
+//              of the faces' common viscous flux (written for both sides);
 //  k_ns_stage  recomputes Q at the solution points, total flux F - F_v, the
-//              common flux = Riemann(U_L, U_R) - F_v(avg U, avg Q).n, FR
+//              common flux = Riemann(U_L, U_R) - (the two shares), FR
 //              correction, stage update and traces of the new state.
+//
+// The common viscous flux F_v(avg U, (Q_L + Q_R)/2).n is linear in the
+// gradient, so it is the sum of F_v(avg U, Q_L/2).n and F_v(avg U, Q_R/2).n.
+// Each side evaluates its share where it has the gradient trace in registers
+// and writes 4 values a flux point instead of the 8 of (dU/dx, dU/dy); the
+// stage kernel adds the own and the neighbour's share (the same sum on both
+// sides), with no viscous evaluation and no gradient data at its faces.
+// Against exchanging the gradients (256 x 256, P3, serialised launches): stage
+// 107 -> 86 us FP64 and 57 -> 54 us FP32, gradient 39 -> 46 and 25 -> 31 us;
+// per step -10.5 % FP64, -4 % FP32 (P5 FP32: -2.5 %).
 //
 // Gradient: U^C = U^D + (U_c - U^D) g at the edges with the common solution
 // U_c = (U_L + U_R)/2 (the ghost state on boundaries), the same VCJH
@@ -41,7 +52,7 @@
 #define ZJ_NSG_MIN_BLOCKS 8       // FP64 point-per-thread gradient kernel
 #endif
 #ifndef ZJ_NS32_MIN_BLOCKS
-#define ZJ_NS32_MIN_BLOCKS 10     // mixed-precision stage kernel (48 registers)
+#define ZJ_NS32_MIN_BLOCKS 8      // mixed-precision stage kernel (64 registers)
 #endif
 #ifndef ZJ_NSG32_MIN_BLOCKS
 #define ZJ_NSG32_MIN_BLOCKS 12    // mixed-precision point-per-thread gradient kernel
@@ -50,13 +61,10 @@
 #define ZJ_NS_MIN_BLOCKS_HI 4     // FP64 stage kernel at P5 (fewer spills)
 #endif
 #ifndef ZJ_NS32_MIN_BLOCKS_HI
-#define ZJ_NS32_MIN_BLOCKS_HI 8   // mixed-precision stage kernel at P5
+#define ZJ_NS32_MIN_BLOCKS_HI 9   // mixed-precision stage kernel at P5 (56 registers)
 #endif
 #ifndef ZJ_NSL_MIN_BLOCKS
-#define ZJ_NSL_MIN_BLOCKS 5       // FP64 gradient kernel by lines (96 registers)
-#endif
-#ifndef ZJ_NSL_MIN_BLOCKS_HI
-#define ZJ_NSL_MIN_BLOCKS_HI 4    // the same from P4 up (no spills)
+#define ZJ_NSL_MIN_BLOCKS 4       // FP64 gradient kernel by lines (128 registers)
 #endif
 #ifndef ZJ_NSL32_MIN_BLOCKS
 #define ZJ_NSL32_MIN_BLOCKS 8     // mixed-precision gradient kernel by lines (64 registers)
@@ -178,6 +186,21 @@ __device__ __forceinline__ void load_face_point(const StageArgsT<T>& a, long lon
     }
 }
 
+// This element's share of the common normal viscous flux of a flux point: Ua
+// the average state, t the own gradient trace, n the face normal.  Half of the
+// flux where a neighbour adds the other half, all of it on a boundary (the
+// ghost gradient is the interior one), with the walls' closure.
+template <typename T>
+__device__ __forceinline__ void viscous_share(const StageArgsT<T>& a, const EdgeRec& r, T nx, T ny,
+                                              const T* Ua, const T* t, T* f) {
+    T Fv[4], Gv[4];
+    viscous_flux_f(Ua, rcp_any(Ua[0]), t, t + 4, T(a.gamma), inv_reynolds(a), T(a.kfac), Fv, Gv);
+    const T w = has_neighbour_gradient(r) ? T(0.5) : T(1);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) f[v] = w * (Fv[v] * nx + Gv[v] * ny);
+    boundary_viscous_closure(r, a.bc, nx, ny, f);
+}
+
 template <int P, typename T>
 __global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS, NSMinBlocks<T, P>::grad)
 k_ns_grad(const StageArgsT<T> a) {
@@ -224,8 +247,8 @@ k_ns_grad(const StageArgsT<T> a) {
 #pragma unroll
         for (int v = 0; v < 4; ++v) { su[v * VS] = u[v]; sut[v * VS] = u[v]; }
     }
+    FacePoint<T> f;
     if (is_fp) {
-        FacePoint<T> f;
         load_face_point<N1>(a, e, edge, fp, f);
         T d[4];
 #pragma unroll
@@ -246,8 +269,14 @@ k_ns_grad(const StageArgsT<T> a) {
         trace_point<N1, RS, VS>(sQ + el * QS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
         trace_point<N1, RS, VS>(sQ + el * QS + 4 * VS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge,
                                 fp, t + 4);
-        T* o = a.TQout + (e * NFT + k) * 8;
-        gstore8(o, t);
+        if (a.GQ) gstore8(a.GQ + (e * NFT + k) * 8, t);
+        if (a.FVout) {
+            T Ua[4], fv[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) Ua[v] = T(0.5) * (f.qo[v] + f.qn[v]);
+            viscous_share(a, f.r, f.nx, f.ny, Ua, t, fv);
+            gstore4(a.FVout + (e * NFT + k) * 4, fv);
+        }
     }
 }
 
@@ -300,7 +329,7 @@ struct LineShape {
     // of a point thread, at half the threads per element.
     // (the counts are per 128 threads; other CTA sizes scale them)
     static constexpr int MIN_BLOCKS_128 =
-        sizeof(T) == 8 ? (P <= 3 ? ZJ_NSL_MIN_BLOCKS : ZJ_NSL_MIN_BLOCKS_HI)
+        sizeof(T) == 8 ? ZJ_NSL_MIN_BLOCKS
                        : (P <= 3 ? ZJ_NSL32_MIN_BLOCKS : ZJ_NSL32_MIN_BLOCKS_HI);
     static constexpr int MIN_BLOCKS = MIN_BLOCKS_128 * 128 / kCtaThreads > 0 ? MIN_BLOCKS_128 * 128 / kCtaThreads : 1;
 };
@@ -350,8 +379,10 @@ k_ns_grad_lines(const StageArgsT<T> a) {
     const int fA = line, fB = N1 - 1 - line;
     constexpr bool kRef = UsesRef<T>::value;
 
-    // jumps U_c - U_own = (U_nbr - U_own)/2 at the line's end points
+    // jumps U_c - U_own = (U_nbr - U_own)/2 and average states at the line's
+    // end points
     T dA[4], dB[4];
+    T UaA[4], UaB[4];
     if (valid) {
 #pragma unroll
         for (int s2 = 0; s2 < 2; ++s2) {
@@ -363,8 +394,12 @@ k_ns_grad_lines(const StageArgsT<T> a) {
             for (int v = 0; v < 4; ++v) qn[v] = qo[v];
             if (!(r.flags & kEdgeOrphan)) load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
             T* d = s2 ? dB : dA;
+            T* m = s2 ? UaB : UaA;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) d[v] = (r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (qn[v] - qo[v]);
+            for (int v = 0; v < 4; ++v) {
+                d[v] = (r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (qn[v] - qo[v]);
+                m[v] = T(0.5) * (qo[v] + qn[v]);
+            }
         }
     }
     cp_async_wait_all();
@@ -447,8 +482,22 @@ k_ns_grad_lines(const StageArgsT<T> a) {
             tB[4 + v] = fma_any(wb, Qy, tB[4 + v]);
         }
     }
-    gstore8(a.TQout + (e * NFT + eA * N1 + fA) * 8, tA);
-    gstore8(a.TQout + (e * NFT + eB * N1 + fB) * 8, tB);
+    if (a.GQ) {
+        gstore8(a.GQ + (e * NFT + eA * N1 + fA) * 8, tA);
+        gstore8(a.GQ + (e * NFT + eB * N1 + fB) * 8, tB);
+    }
+    if (!a.FVout) return;
+#pragma unroll
+    for (int s2 = 0; s2 < 2; ++s2) {
+        const int ed = s2 ? eB : eA, fp = s2 ? fB : fA;
+        // (read again here: held from the jumps on, they cost more in
+        // registers than the second L1 access)
+        const EdgeRec r = a.edges[e * 4 + ed];
+        T n[3], f[4];
+        load_normal(normal_rec<N1>(a, e, ed, fp), n);
+        viscous_share(a, r, n[0], n[1], s2 ? UaB : UaA, s2 ? tB : tA, f);
+        gstore4(a.FVout + (e * NFT + ed * N1 + fp) * 4, f);
+    }
 }
 
 template <int P, int RIEM, typename T>
@@ -466,16 +515,11 @@ k_ns_stage(const StageArgsT<T> a) {
     __shared__ __align__(16) T sD[EB * DS];   // face jumps of U, then flux differences
     __shared__ __align__(16) T sU[EB * FS];   // stage state, then the new state
     __shared__ double sRed[32];
-    // A flux-point thread's face data from the loads to the face phase, parked
-    // here (component-major: a warp's accesses fill consecutive banks) so
-    // that it holds no registers through the volume phase: own and neighbour
-    // traces (4 + 4) and the average gradient trace (8).
-    __shared__ T sFP[16 * S::THREADS];
 
     const int tid = threadIdx.x;
     for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
     pdl_launch_dependents();
-    pdl_wait();   // the gradient traces come from k_ns_grad, the state from the previous stage
+    pdl_wait();   // the viscous shares come from the gradient launch, the state from the previous stage
     const int el = tid / TPE, k = tid - el * TPE;
     bool valid;
     const long long e = block_element(a, EB, el, valid);
@@ -484,36 +528,15 @@ k_ns_stage(const StageArgsT<T> a) {
     const int edge = k / N1, fp = k - edge * N1;
     const int i = k % N1, j = k / N1;
 
-    // ---- A1: loads, face jumps, stage state into shared memory
+    // ---- A1: loads, face jumps, stage state into shared memory; the common
+    // flux of the flux points, which needs nothing else (a thread carries its
+    // four values, not the traces they came from, through the volume phase)
     FacePoint<T> f;
-    T* pk = sFP + tid;   // this thread's parked face data, stride S::THREADS
-    if (is_fp) {
-        T Qo[8], Qn[8];
-        load_face_point<N1>(a, e, edge, fp, f);
-        const T* qt = a.TQ + (e * NFT + k) * 8;
-        gload8_nc(qt, Qo);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) Qn[v] = Qo[v];
-        if (has_neighbour_gradient(f.r)) {
-            const T* qn = a.TQ + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 8;
-            gload8_nc(qn, Qn);
-        }
-        T d[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) d[v] = (f.r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (f.qn[v] - f.qo[v]);
-        store4(sD + el * DS + k * 4, d);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            pk[v * S::THREADS] = f.qo[v];
-            pk[(4 + v) * S::THREADS] = f.qn[v];
-        }
-#pragma unroll
-        for (int v = 0; v < 8; ++v) pk[(8 + v) * S::THREADS] = T(0.5) * (Qo[v] + Qn[v]);
-    }
     constexpr bool kRef = UsesRef<T>::value;
     T ue[4] = {T(0), T(0), T(0), T(0)};   // reference state (mixed form)
     if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
     T u[4], ji[4], Jd = T(1);
+    T Fd[4] = {T(0), T(0), T(0), T(0)};
     if (is_sp) {
         const long long idx = e * NSP + k;
         double ud[4];
@@ -530,6 +553,34 @@ k_ns_stage(const StageArgsT<T> a) {
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) su[v * VS] = w[v];
+    }
+    if (is_fp) {
+        T fo[4], fn[4] = {T(0), T(0), T(0), T(0)};
+        load_face_point<N1>(a, e, edge, fp, f);
+        load4_nc(a.FV + (e * NFT + k) * 4, fo);
+        if (has_neighbour_gradient(f.r))
+            load4_nc(a.FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
+        T d[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) d[v] = (f.r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (f.qn[v] - f.qo[v]);
+        store4(sD + el * DS + k * 4, d);
+        if (!(f.r.flags & kEdgeOrphan)) {
+            // evaluated from the left element's side on both sides
+            const bool right = (f.r.flags & kEdgeRight) != 0;
+            T UL[4], UR[4], Fc[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) { UL[v] = right ? f.qn[v] : f.qo[v]; UR[v] = right ? f.qo[v] : f.qn[v]; }
+            riemann<RIEM>(UL, UR, f.nx, f.ny, g, Fc);
+            if constexpr (kRef) {
+                T Fe[4];
+                ref_flux_n(ue, g, f.nx, f.ny, Fe);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
+            }
+            const T ss = right ? T(-0.5) * f.len : T(0.5) * f.len;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) Fd[v] = ss * (Fc[v] - (fo[v] + fn[v]));
+        }
     }
     __syncthreads();
 
@@ -560,39 +611,9 @@ k_ns_stage(const StageArgsT<T> a) {
     }
     __syncthreads();   // face jumps and the stage state in shared memory are dead now
 
-    // ---- B: interface terms, evaluated from the left element's side
+    // ---- B: flux differences at the faces
     if (is_fp) {
-        T Fd[4] = {T(0), T(0), T(0), T(0)};
         if (!(f.r.flags & kEdgeOrphan)) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                f.qo[v] = pk[v * S::THREADS];
-                f.qn[v] = pk[(4 + v) * S::THREADS];
-            }
-            const bool right = (f.r.flags & kEdgeRight) != 0;
-            T UL[4], UR[4], Fc[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) { UL[v] = right ? f.qn[v] : f.qo[v]; UR[v] = right ? f.qo[v] : f.qn[v]; }
-            riemann<RIEM>(UL, UR, f.nx, f.ny, g, Fc);
-            if constexpr (kRef) {
-                T Fe[4];
-                ref_flux_n(ue, g, f.nx, f.ny, Fe);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
-            }
-            T Ua[4], dxa[4], dya[4], Fv[4], Gv[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                Ua[v] = T(0.5) * (UL[v] + UR[v]);
-                dxa[v] = pk[(8 + v) * S::THREADS];
-                dya[v] = pk[(12 + v) * S::THREADS];
-            }
-            viscous_flux_f(Ua, rcp_any(Ua[0]), dxa, dya, g, inv_reynolds(a), T(a.kfac), Fv, Gv);
-            T Fvn[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) Fvn[v] = Fv[v] * f.nx + Gv[v] * f.ny;
-            boundary_viscous_closure(f.r, a.bc, f.nx, f.ny, Fvn);
-            const T ss = right ? T(-0.5) * f.len : T(0.5) * f.len;
             const bool along_eta = (edge == 0 || edge == 2);
             T Fn[4];
             if constexpr (kTrG)
@@ -604,8 +625,7 @@ k_ns_stage(const StageArgsT<T> a) {
                                         sOps + N1 * N1 + N1, edge, fp, Fn);
             const T sgn = (edge == 0 || edge == 3) ? T(-1) : T(1);
 #pragma unroll
-            for (int v = 0; v < 4; ++v)
-                Fd[v] = ss * (Fc[v] - Fvn[v]) - sgn * Fn[v];
+            for (int v = 0; v < 4; ++v) Fd[v] -= sgn * Fn[v];
         }
         store4(sD + el * DS + k * 4, Fd);
     }

@@ -145,16 +145,15 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
     // ---- A1: loads, face jumps, stage state into shared memory
     FacePoint<float> f;
     f.r = EdgeRec{-1, 0, kEdgeOrphan, 0};
-    float Qo[8], Qn[8];
+    float fv[4] = {0.f, 0.f, 0.f, 0.f};   // common normal viscous flux: both sides' shares
     if (is_fp) {
         load_face_point<N1>(a, e, edge, fp, f);
-        const float* qt = a.TQ + (e * NFT + k) * 8;
-        gload8_nc(qt, Qo);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) Qn[v] = Qo[v];
+        load4_nc(a.FV + (e * NFT + k) * 4, fv);
         if (has_neighbour_gradient(f.r)) {
-            const float* qn = a.TQ + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 8;
-            gload8_nc(qn, Qn);
+            float fn[4];
+            load4_nc(a.FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) fv[v] += fn[v];
         }
         float d[4];
 #pragma unroll
@@ -244,21 +243,8 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
         riemann<RIEM>(UL, UR, f.nx, f.ny, g, Fc);
         float Fe[4];
         ref_flux_n(ue, g, f.nx, f.ny, Fe);
-        float Ua[4], dxa[4], dya[4], Fv[4], Gv[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            Fc[v] -= Fe[v];
-            Ua[v] = 0.5f * (UL[v] + UR[v]);
-            dxa[v] = 0.5f * (Qo[v] + Qn[v]);
-            dya[v] = 0.5f * (Qo[4 + v] + Qn[4 + v]);
-        }
-        viscous_flux_f(Ua, rcp_any(Ua[0]), dxa, dya, g, inv_reynolds(a), float(a.kfac), Fv, Gv);
-        float Fvn[4];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) Fvn[v] = Fv[v] * f.nx + Gv[v] * f.ny;
-        boundary_viscous_closure(f.r, a.bc, f.nx, f.ny, Fvn);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) Fc[v] -= Fvn[v];
+        for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v] + fv[v];
     }
 
     // ---- the product: tensor memory -> the result tile (rows 16q..16q+15 sit

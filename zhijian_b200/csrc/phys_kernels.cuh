@@ -98,7 +98,7 @@ __device__ __forceinline__ long long neighbour_row(const EdgeRec& r, long long n
 __device__ __forceinline__ bool boundary_condition_edge(const EdgeRec& r) {
     return (r.flags & (kEdgeBoundary | kEdgeInterface)) == kEdgeBoundary;
 }
-// An edge whose neighbour's gradient trace is read (interior edges and
+// An edge whose neighbour's viscous share is read (interior edges and
 // partition interfaces; a boundary copies the interior gradient).
 __device__ __forceinline__ bool has_neighbour_gradient(const EdgeRec& r) {
     return !(r.flags & kEdgeOrphan) && (!(r.flags & kEdgeBoundary) || (r.flags & kEdgeInterface));
@@ -152,12 +152,6 @@ __device__ __forceinline__ void store_residual(const StageArgsT<T>& a, long long
         for (int v = 0; v < 4; ++v) td[v] = res[v].d;
         gstore4(a.dR + idx * 4, td);
     }
-}
-
-template <typename T>
-__device__ __forceinline__ T reynolds(const StageArgsT<T>& a) {
-    if constexpr (IsDual<T>::value) return Dual(a.Re, a.dRe);
-    else return T(a.Re);
 }
 
 // 1/Re (with its tangent -dRe/Re^2 for duals) and gamma/((gamma-1) Pr),

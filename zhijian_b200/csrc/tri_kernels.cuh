@@ -194,15 +194,20 @@ k_tri_grad(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n
 #pragma unroll
         for (int v = 0; v < 4; ++v) sU[el * ES + v * FS + k] = u[v];
     }
+    EdgeRec r{-1, 0, kEdgeOrphan, 0};
+    T Ua[4];   // average state of the flux point
     if (is_fp) {
-        const EdgeRec r = a.edges[e * 4 + edge];
-        T qo[4], qn[4];
-        load4_nc(a.Tin + (e * 4 * N1 + k) * 4, qo);
+        r = a.edges[e * 4 + edge];
+        T qn[4];
+        load4_nc(a.Tin + (e * 4 * N1 + k) * 4, Ua);
         T d[4] = {T(0), T(0), T(0), T(0)};
         if (!(r.flags & kEdgeOrphan)) {
             load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) d[v] = T(0.5) * (qn[v] - qo[v]);
+            for (int v = 0; v < 4; ++v) {
+                d[v] = T(0.5) * (qn[v] - Ua[v]);
+                Ua[v] = T(0.5) * (Ua[v] + qn[v]);
+            }
         }
         store4(sDU + el * DS + k * 4, d);
     }
@@ -222,8 +227,10 @@ k_tri_grad(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n
         T t[8];
         tri_interp<NT, FS>(sQ + el * 2 * ES, sOps + Lo::L + k * NT, t);
         tri_interp<NT, FS>(sQ + el * 2 * ES + ES, sOps + Lo::L + k * NT, t + 4);
-        T* o = a.TQout + (e * 4 * N1 + k) * 8;
-        gstore8(o, t);
+        T n[3], f[4];
+        load_normal(a.enrm + e * 4 + edge, n);
+        viscous_share(a, r, n[0], n[1], Ua, t, f);
+        gstore4(a.FVout + (e * 4 * N1 + k) * 4, f);
     }
 }
 
@@ -250,7 +257,7 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
     const bool valid = e >= 0;
     const bool is_sp = valid && k < NT, is_fp = valid && k < NFT;
     const int edge = k / N1, fp = k - edge * N1;
-    const T g = T(a.gamma), Re = reynolds(a), Pr = T(a.Pr);
+    const T g = T(a.gamma);
     constexpr bool kRef = UsesRef<T>::value;
 
     // ---- A1: loads
@@ -258,7 +265,7 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
     if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
     T nr[3] = {T(0), T(0), T(0)}, qo[4], qn[4] = {T(0), T(0), T(0), T(0)};
-    T Qo[8], Qn[8];
+    T fv[4] = {T(0), T(0), T(0), T(0)};   // common normal viscous flux: both sides' shares
     if (is_fp) {
         r = a.edges[e * 4 + edge];
         load_normal(a.enrm + e * 4 + edge, nr);
@@ -267,13 +274,12 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
         for (int v = 0; v < 4; ++v) qn[v] = qo[v];
         if (!(r.flags & kEdgeOrphan)) load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
         if constexpr (VISC) {
-            const T* qt = a.TQ + (e * 4 * N1 + k) * 8;
-            gload8_nc(qt, Qo);
-#pragma unroll
-            for (int v = 0; v < 8; ++v) Qn[v] = Qo[v];
+            load4_nc(a.FV + (e * 4 * N1 + k) * 4, fv);
             if (!(r.flags & (kEdgeOrphan | kEdgeBoundary))) {
-                const T* q2 = a.TQ + (((long long)r.nbr * 4 + r.nbr_edge) * N1 + (N1 - 1 - fp)) * 8;
-                gload8_nc(q2, Qn);
+                T fn[4];
+                load4_nc(a.FV + (((long long)r.nbr * 4 + r.nbr_edge) * N1 + (N1 - 1 - fp)) * 4, fn);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) fv[v] += fn[v];
             }
             T d[4];
 #pragma unroll
@@ -316,7 +322,7 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
             T Qx[4], Qy[4], Fv[4], Gv[4];
             tri_gradient<NT, NFT, FS>(sU + el * ES, sD + el * DS, sOps + Lo::DR, sOps + Lo::DSo, sOps + Lo::PHI,
                                       k, ji, Qx, Qy);
-            viscous_flux(u, Qx, Qy, g, Re, Pr, Fv, Gv);
+            viscous_flux_f(u, rcp_any(u[0]), Qx, Qy, g, inv_reynolds(a), T(a.kfac), Fv, Gv);
 #pragma unroll
             for (int v = 0; v < 4; ++v) { F[v] -= Fv[v]; G[v] -= Gv[v]; }
         }
@@ -344,20 +350,8 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
                 for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
             }
             if constexpr (VISC) {
-                T Ua[4], dxa[4], dya[4], Fv[4], Gv[4];
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    Ua[v] = T(0.5) * (UL[v] + UR[v]);
-                    dxa[v] = T(0.5) * (Qo[v] + Qn[v]);
-                    dya[v] = T(0.5) * (Qo[4 + v] + Qn[4 + v]);
-                }
-                viscous_flux(Ua, dxa, dya, g, Re, Pr, Fv, Gv);
-                T Fvn[4];
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Fvn[v] = Fv[v] * nr[0] + Gv[v] * nr[1];
-                boundary_viscous_closure(r, a.bc, nr[0], nr[1], Fvn);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Fc[v] -= Fvn[v];
+                for (int v = 0; v < 4; ++v) Fc[v] -= fv[v];
             }
             const T sf = nr[2] * T(1.0 / tri_ref_len(edge));
             const T ss = right ? -sf : sf;

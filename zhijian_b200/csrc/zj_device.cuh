@@ -74,10 +74,6 @@ __device__ __forceinline__ void gstore4(double* p, const double* v) {
                  : "memory");
 }
 // Eight values (a gradient-trace point): two 32-byte accesses.
-__device__ __forceinline__ void gload8_nc(const double* p, double* v) {
-    load4_nc(p, v);
-    load4_nc(p + 4, v + 4);
-}
 __device__ __forceinline__ void gstore8(double* p, const double* v) {
     gstore4(p, v);
     gstore4(p + 4, v + 4);
@@ -102,11 +98,6 @@ __device__ __forceinline__ void store4(float* p, const float* v) {
 // Global float rows: four values are one 16-byte access; eight (a gradient
 // trace point, 32-byte aligned like the double rows) one 32-byte access.
 __device__ __forceinline__ void gstore4(float* p, const float* v) { store4(p, v); }
-__device__ __forceinline__ void gload8_nc(const float* p, float* v) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-        : "l"(p));
-}
 __device__ __forceinline__ void gstore8(float* p, const float* v) {
     asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
                  "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])

@@ -93,10 +93,6 @@ __device__ __forceinline__ void store4(Dual* p, const Dual* v) {
 // The global-row helpers of the FP64 and FP32 kernels, on dual numbers.
 __device__ __forceinline__ void gload4(const Dual* p, Dual* v) { load4(p, v); }
 __device__ __forceinline__ void gstore4(Dual* p, const Dual* v) { store4(p, v); }
-__device__ __forceinline__ void gload8_nc(const Dual* p, Dual* v) {
-    load4(p, v);
-    load4(p + 4, v + 4);
-}
 __device__ __forceinline__ void gstore8(Dual* p, const Dual* v) {
     store4(p, v);
     store4(p + 4, v + 4);

@@ -40,8 +40,11 @@ struct StageArgsT {
     double gamma;
     int stage;              // 0: residual only; 1..3: SSP-RK3 stage
     // Navier-Stokes
-    const T* TQ;            // gradient traces of U, [E][4 edges][n1][8] = (dU/dx, dU/dy)
-    T* TQout;               // gradient traces written by the gradient launch
+    const T* FV;            // this side's share of the common normal viscous flux at every flux
+                            // point, [E][4 edges][n1][4] (then a partition's interface rows)
+    T* FVout;               // the same, written by the gradient launch
+    T* GQ;                  // gradient traces (dU/dx, dU/dy), [E][4 edges][n1][8], also written by
+                            // the gradient launch when not NULL (the adjoint reads them)
     double Re, Pr;
     double iRe, kfac;       // 1/Re and gamma/((gamma-1) Pr) of the viscosity law
     int* tc_err;            // split-BF16 kernel: set to 1 if a bounded wait gave up

@@ -261,31 +261,10 @@ __device__ __forceinline__ void ghost_phys(const T* Ui, T nx, T ny, int bct,
 // Viscous flux of the reference's computeViscousFluxSPKernel
 // (kernels.cu:742-786): velocity and temperature gradients from the
 // conservative gradients dx = dU/dx, dy = dU/dy; mu = T^0.7/Re,
-// k = mu gamma / ((gamma-1) Pr); Stokes hypothesis.
-template <typename T>
-__device__ __forceinline__ void viscous_flux(const T* s, const T* dx, const T* dy, T g, T Re,
-                                             T Pr, T* Fv, T* Gv) {
-    const T ir = rcp_any(s[0]);
-    const T u = s[1] * ir, v = s[2] * ir;
-    const T dudx = (dx[1] - u * dx[0]) * ir, dudy = (dy[1] - u * dy[0]) * ir;
-    const T dvdx = (dx[2] - v * dx[0]) * ir, dvdy = (dy[2] - v * dy[0]) * ir;
-    const T p = (g - T(1)) * s[0] * (s[3] * ir - T(0.5) * (u * u + v * v));
-    const T Tm = p * ir;
-    const T dpdx = (g - T(1)) * (dx[3] - T(0.5) * dx[0] * (u * u + v * v) - s[0] * (u * dudx + v * dvdx));
-    const T dpdy = (g - T(1)) * (dy[3] - T(0.5) * dy[0] * (u * u + v * v) - s[0] * (u * dudy + v * dvdy));
-    const T dTdx = (dpdx - Tm * dx[0]) * ir, dTdy = (dpdy - Tm * dy[0]) * ir;
-    const T mu = div_any(visc_pow(Tm), Re);
-    const T k = div_any(mu * g, (g - T(1)) * Pr);
-    const T div = dudx + dvdy, lam = T(-2.0 / 3.0) * mu;
-    const T txx = T(2) * mu * dudx + lam * div, tyy = T(2) * mu * dvdy + lam * div;
-    const T txy = mu * (dudy + dvdx);
-    Fv[0] = T(0); Fv[1] = txx; Fv[2] = txy; Fv[3] = u * txx + v * txy + k * dTdx;
-    Gv[0] = T(0); Gv[1] = txy; Gv[2] = tyy; Gv[3] = u * txy + v * tyy + k * dTdy;
-}
-
-// viscous_flux with ir = 1/s[0] supplied and the law's two divisions taken
-// as products with iRe = 1/Re and kfac = gamma/((gamma-1) Pr), computed once
-// per thread (each within 2 ulp of the divided form).
+// k = mu gamma / ((gamma-1) Pr); Stokes hypothesis.  ir = 1/s[0] is the
+// caller's, and the law's two divisions are products with iRe = 1/Re and
+// kfac = gamma/((gamma-1) Pr), computed once per launch (each within 2 ulp of
+// the divided form).
 template <typename T>
 __device__ __forceinline__ void viscous_flux_f(const T* s, T ir, const T* dx, const T* dy, T g, T iRe,
                                                T kfac, T* Fv, T* Gv) {
