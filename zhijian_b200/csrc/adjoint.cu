@@ -80,6 +80,34 @@ __device__ __forceinline__ void transposed_divergence(const double* sA, const do
     }
 }
 
+// Corrected gradient at solution point (i, j): su the state tile
+// [var][row][col], du the face jumps in the flux-point tile.
+template <int P, int RS, int VS>
+__device__ __forceinline__ void corrected_gradient_vars(const double* su, const double* du, const double* ops, int i,
+                                                        int j, const double* ji, double* Qx, double* Qy) {
+    constexpr int N1 = P + 1;
+    const double* gL = ops + N1 * N1 + 2 * N1;
+    const double* gR = gL + N1;
+    double d1[4], d3[4], d0[4], d2[4];
+    load4(du + face_slot<P, double>(1, 1, j), d1);
+    load4(du + face_slot<P, double>(1, 0, j), d3);
+    load4(du + face_slot<P, double>(0, 0, i), d0);
+    load4(du + face_slot<P, double>(0, 1, i), d2);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        double dxi = 0.0, deta = 0.0;
+#pragma unroll
+        for (int m = 0; m < N1; ++m) {
+            dxi = fma(ops[i * N1 + m], su[v * VS + j * RS + m], dxi);
+            deta = fma(ops[j * N1 + m], su[v * VS + m * RS + i], deta);
+        }
+        dxi += gR[i] * d1[v] + gL[i] * d3[v];
+        deta += gL[j] * d0[v] + gR[j] * d2[v];
+        Qx[v] = ji[0] * dxi + ji[2] * deta;
+        Qy[v] = ji[1] * dxi + ji[3] * deta;
+    }
+}
+
 // L^T of the four edges' trace adjoints at solution point (i, j), added to
 // out: W values per flux point, flux point k at sT + k * stride.
 template <int N1, int W>
@@ -232,7 +260,8 @@ k_adj_ns(const AdjArgs a) {
     __shared__ double sOps[S::NOPS];
     __shared__ __align__(16) double sA[EB * FS];      // a, then dxi-bar
     __shared__ __align__(16) double sU[EB * FS];      // stage state, then deta-bar
-    __shared__ __align__(16) double sD[EB * DS];      // face jumps of U
+    constexpr int DJ = Tiles<P, double>::DP;
+    __shared__ __align__(16) double sD[EB * DJ];      // face jumps of U
     __shared__ __align__(16) double sDF[EB * DS];     // own dFbar
     __shared__ __align__(16) double sTQ[EB * 2 * DS]; // own gradient-trace adjoint
     __shared__ double sRed[32];
@@ -278,7 +307,8 @@ k_adj_ns(const AdjArgs a) {
         double d[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) d[v] = (r.flags & kEdgeOrphan) ? 0.0 : 0.5 * (qn[v] - qo[v]);
-        store4(sD + el * DS + k * 4, d);
+        const int dir = edge & 1, side = (edge == 1 || edge == 2);
+        store4(sD + el * DJ + face_slot<P, double>(dir, side, (dir == side) ? fp : N1 - 1 - fp), d);
     }
     double u[4], ji[4], Jd = 1.0;
     if (is_sp) {
@@ -297,7 +327,7 @@ k_adj_ns(const AdjArgs a) {
     double ub[4] = {0.0, 0.0, 0.0, 0.0}, Qxb[4] = {0.0, 0.0, 0.0, 0.0}, Qyb[4] = {0.0, 0.0, 0.0, 0.0};
     if (is_sp) {
         double Qx[4], Qy[4];
-        corrected_gradient<N1, RS, VS>(sU + el * FS, sD + el * DS, sOps, i, j, ji, Qx, Qy);
+        corrected_gradient_vars<P, RS, VS>(sU + el * FS, sD + el * DJ, sOps, i, j, ji, Qx, Qy);
         double Ftb[4], Gtb[4], Fb[4], Gb[4], mFb[4], mGb[4];
         transposed_divergence<N1, RS, VS>(sA + el * FS, sDF + el * DS, sOps, i, j, Ftb, Gtb);
 #pragma unroll

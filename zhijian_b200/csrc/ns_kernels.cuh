@@ -46,7 +46,7 @@
 // Resident CTAs per SM the launch bounds ask for, counted in CTAs of 128
 // threads (other CTA sizes scale them).
 #ifndef ZJ_NS_MIN_BLOCKS
-#define ZJ_NS_MIN_BLOCKS 5        // FP64 stage kernel (96 registers)
+#define ZJ_NS_MIN_BLOCKS 4        // FP64 stage kernel (128 registers)
 #endif
 #ifndef ZJ_NSG_MIN_BLOCKS
 #define ZJ_NSG_MIN_BLOCKS 8       // FP64 point-per-thread gradient kernel
@@ -56,12 +56,6 @@
 #endif
 #ifndef ZJ_NSG32_MIN_BLOCKS
 #define ZJ_NSG32_MIN_BLOCKS 12    // mixed-precision point-per-thread gradient kernel
-#endif
-#ifndef ZJ_NS_MIN_BLOCKS_HI
-#define ZJ_NS_MIN_BLOCKS_HI 4     // FP64 stage kernel at P5 (fewer spills)
-#endif
-#ifndef ZJ_NS32_MIN_BLOCKS_HI
-#define ZJ_NS32_MIN_BLOCKS_HI 9   // mixed-precision stage kernel at P5 (56 registers)
 #endif
 #ifndef ZJ_NSL_MIN_BLOCKS
 #define ZJ_NSL_MIN_BLOCKS 4       // FP64 gradient kernel by lines (128 registers)
@@ -82,86 +76,46 @@ using namespace phys;
 template <typename T, int P> struct NSMinBlocks;
 constexpr int per_cta(int blocks128) { return blocks128 * 128 / kCtaThreads > 0 ? blocks128 * 128 / kCtaThreads : 1; }
 template <int P> struct NSMinBlocks<double, P> {
-    static constexpr int stage = per_cta(P <= 4 ? ZJ_NS_MIN_BLOCKS : ZJ_NS_MIN_BLOCKS_HI);
+    static constexpr int stage = per_cta(ZJ_NS_MIN_BLOCKS);
     static constexpr int grad = per_cta(ZJ_NSG_MIN_BLOCKS);
 };
 template <int P> struct NSMinBlocks<float, P> {
-    static constexpr int stage = per_cta(P <= 4 ? ZJ_NS32_MIN_BLOCKS : ZJ_NS32_MIN_BLOCKS_HI);
+    static constexpr int stage = per_cta(ZJ_NS32_MIN_BLOCKS);
     static constexpr int grad = per_cta(ZJ_NSG32_MIN_BLOCKS);
 };
 template <int P> struct NSMinBlocks<Dual, P> { static constexpr int stage = 1, grad = 1; };
 
 // Corrected gradient at solution point (i, j) of one element: su is the
-// element's state in the [var][row][col] shared layout, du its face jumps
-// U_c - U_own in the [flux point][var] layout.
-template <int N1, int RS, int VS, typename T>
-__device__ __forceinline__ void corrected_gradient(const T* su, const T* du, const T* ops, int i,
+// element's state tile, du its face jumps U_c - U_own in the flux-point tile.
+template <int P, typename T>
+__device__ __forceinline__ void corrected_gradient(const T* su, const T* du, const Weight<T>* ops, int i,
                                                    int j, const T* ji, T* Qx, T* Qy) {
-    const T* gL = ops + N1 * N1 + 2 * N1;
-    const T* gR = gL + N1;
-    T Di[N1], Dj[N1];
-#pragma unroll
-    for (int m = 0; m < N1; ++m) { Di[m] = ops[i * N1 + m]; Dj[m] = ops[j * N1 + m]; }
-    T d1[4], d3[4], d0[4], d2[4];
-    load4(du + (1 * N1 + j) * 4, d1);
-    load4(du + (3 * N1 + (N1 - 1 - j)) * 4, d3);
-    load4(du + (0 * N1 + i) * 4, d0);
-    load4(du + (2 * N1 + (N1 - 1 - i)) * 4, d2);
-    const T gRi = gR[i], gLi = gL[i], gRj = gR[j], gLj = gL[j];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        T row[N1];
-        load_row<N1>(su + v * VS + j * RS, row);
-        T dxi = T(0), deta = T(0);
-#pragma unroll
-        for (int m = 0; m < N1; ++m) {
-            dxi = fma_any(Di[m], row[m], dxi);
-            deta = fma_any(Dj[m], su[v * VS + m * RS + i], deta);
-        }
-        dxi += gRi * d1[v] + gLi * d3[v];
-        deta += gLj * d0[v] + gRj * d2[v];
-        Qx[v] = ji[0] * dxi + ji[2] * deta;
-        Qy[v] = ji[1] * dxi + ji[3] * deta;
-    }
+    using Op = OpTable<P + 1, T>;
+    constexpr int N1 = P + 1, RP = Tiles<P, T>::RP;
+    Weight<T> w[N1];
+    load_weights<N1>(ops + i * N1, w);
+    V4<T> dxi = line_dot<N1>(w, su + j * RP, 4, v4_zero<T>());
+    dxi = v4_fma(ops[Op::GR + i], v4_load(du + face_slot<P, T>(1, 1, j)), dxi);
+    dxi = v4_fma(ops[Op::GL + i], v4_load(du + face_slot<P, T>(1, 0, j)), dxi);
+    load_weights<N1>(ops + j * N1, w);
+    V4<T> deta = line_dot<N1>(w, su + 4 * i, RP, v4_zero<T>());
+    deta = v4_fma(ops[Op::GL + j], v4_load(du + face_slot<P, T>(0, 0, i)), deta);
+    deta = v4_fma(ops[Op::GR + j], v4_load(du + face_slot<P, T>(0, 1, i)), deta);
+    v4_get(v4_fma(weight<T>(ji[2]), deta, v4_mul(weight<T>(ji[0]), dxi)), Qx);
+    v4_get(v4_fma(weight<T>(ji[3]), deta, v4_mul(weight<T>(ji[1]), dxi)), Qy);
 }
 
-// The same gradient with the element's tile also held transposed (sut:
-// [var][xi][eta]), so the eta-line of point (i, j) is a row: vector loads
-// instead of N1 strided ones; the sums run in the same order.
-template <int N1, int RS, int VS, typename T>
-__device__ __forceinline__ void corrected_gradient_tr(const T* su, const T* sut, const T* du, const T* ops,
-                                                      int i, int j, const T* ji, T* Qx, T* Qy) {
-    const T* gL = ops + N1 * N1 + 2 * N1;
-    const T* gR = gL + N1;
-    T Di[N1], Dj[N1];
-#pragma unroll
-    for (int m = 0; m < N1; ++m) { Di[m] = ops[i * N1 + m]; Dj[m] = ops[j * N1 + m]; }
-    T d1[4], d3[4], d0[4], d2[4];
-    load4(du + (1 * N1 + j) * 4, d1);
-    load4(du + (3 * N1 + (N1 - 1 - j)) * 4, d3);
-    load4(du + (0 * N1 + i) * 4, d0);
-    load4(du + (2 * N1 + (N1 - 1 - i)) * 4, d2);
-    const T gRi = gR[i], gLi = gL[i], gRj = gR[j], gLj = gL[j];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        T row[N1], col[N1];
-        load_row<N1>(su + v * VS + j * RS, row);
-        load_row<N1>(sut + v * VS + i * RS, col);
-        T dxi = T(0), deta = T(0);
-#pragma unroll
-        for (int m = 0; m < N1; ++m) {
-            dxi = fma_any(Di[m], row[m], dxi);
-            deta = fma_any(Dj[m], col[m], deta);
-        }
-        dxi += gRi * d1[v] + gLi * d3[v];
-        deta += gLj * d0[v] + gRj * d2[v];
-        Qx[v] = ji[0] * dxi + ji[2] * deta;
-        Qy[v] = ji[1] * dxi + ji[3] * deta;
-    }
+// A load of the stage kernel: in its place in FP32, the compiler's to place
+// in FP64 and for dual numbers (see the load phase of k_ns_stage).
+template <typename T>
+__device__ __forceinline__ void load4_x(const T* p, T* v) {
+    if constexpr (sizeof(T) == 4) load4_now(p, v);
+    else load4_nc(p, v);
 }
 
-// Loads of a flux-point thread: edge record, normal, own trace, the
-// neighbour's coinciding trace point or the ghost state.
+// Loads of a flux-point thread: edge record, normal, own trace; then the
+// neighbour's coinciding trace point (interior) or the ghost row written with
+// the trace (boundary).  Tin: the stage's traces, behind the wait.
 template <typename T>
 struct FacePoint {
     EdgeRec r;
@@ -170,20 +124,19 @@ struct FacePoint {
 };
 
 template <int N1, typename T>
-__device__ __forceinline__ void load_face_point(const StageArgsT<T>& a, long long e, int edge, int fp,
-                                                FacePoint<T>& f) {
-    constexpr int NFT = 4 * N1;
+__device__ __forceinline__ void load_own_face(const StageArgsT<T>& a, const T* Tin, long long e, int edge, int fp,
+                                              FacePoint<T>& f) {
     f.r = a.edges[e * 4 + edge];
     T n[3];
     load_normal(normal_rec<N1>(a, e, edge, fp), n);
     f.nx = n[0]; f.ny = n[1]; f.len = n[2];
-    load4_nc(a.Tin + (e * NFT + edge * N1 + fp) * 4, f.qo);
+    load4_x(Tin + (e * 4 * N1 + edge * N1 + fp) * 4, f.qo);
+}
+
+template <int N1, typename T>
+__device__ __forceinline__ void load_neighbour_face(const StageArgsT<T>& a, const T* Tin, int fp, FacePoint<T>& f) {
     f.qn[0] = f.qo[0]; f.qn[1] = f.qo[1]; f.qn[2] = f.qo[2]; f.qn[3] = f.qo[3];
-    if (!(f.r.flags & kEdgeOrphan)) {
-        // interior: the neighbour's coinciding point; boundary: the ghost row
-        // written with the trace
-        load4_nc(a.Tin + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, f.qn);
-    }
+    if (!(f.r.flags & kEdgeOrphan)) load4_x(Tin + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, f.qn);
 }
 
 // This element's share of the common normal viscous flux of a flux point: Ua
@@ -206,29 +159,31 @@ __global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS, NSMinBlock
 k_ns_grad(const StageArgsT<T> a) {
     using S = Shape<P, EbDiv<T>::value>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = Tiles<P, T>::FS, DS = Tiles<P, T>::DS;
-    constexpr int QS = Tiles<P, T>::QS;
-    __shared__ T sOps[S::NOPS];
-    __shared__ __align__(16) T sU[EB * FS];
-    __shared__ __align__(16) T sUt[EB * FS];   // the same tile transposed
-    __shared__ __align__(16) T sDU[EB * DS];
-    __shared__ __align__(16) T sQ[EB * QS];
+    using Op = OpTable<P + 1, T>;
+    constexpr int RP = Tiles<P, T>::RP, FP = Tiles<P, T>::FP, DP = Tiles<P, T>::DP;
+    __shared__ __align__(16) Weight<T> sOps[Op::N];
+    __shared__ __align__(16) T sU[EB * FP];
+    __shared__ __align__(16) T sDU[EB * DP];
+    __shared__ __align__(16) T sQx[EB * FP];
+    __shared__ __align__(16) T sQy[EB * FP];
 
     const int tid = threadIdx.x;
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    Op::fill(sOps, a.ops);
     pdl_launch_dependents();
     pdl_wait();   // the state and traces come from the previous stage
     const int el = tid / TPE, k = tid - el * TPE;
     bool valid;
     const long long e = block_element(a, EB, el, valid);
     const bool is_sp = valid && k < NSP, is_fp = valid && k < NFT;
-    const int edge = k / N1, fp = k - edge * N1;
-    const int i = k % N1, j = k / N1;
+    const FaceLane fl = lane_face<N1>(k);
+    const int edge = fl.edge, fp = fl.fp, kf = edge * N1 + fp;
+    int i, j;
+    lane_point<N1>(k, i, j);
 
     constexpr bool kRef = UsesRef<T>::value;
     T ji[4];
     if (is_sp) {
-        const long long idx = e * NSP + k;
+        const long long idx = e * NSP + j * N1 + i;
         T u[4];
         if constexpr (kRef) {
             // D (U - U_e): the reference drops out of the derivative exactly
@@ -242,40 +197,37 @@ k_ns_grad(const StageArgsT<T> a) {
             stage_state(a, idx, ud, u);
         }
         load4_nc(a.Jinv + idx * 4, ji);
-        T* su = sU + el * FS + j * RS + i;
-        T* sut = sUt + el * FS + i * RS + j;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) { su[v * VS] = u[v]; sut[v * VS] = u[v]; }
+        store4(sU + el * FP + j * RP + 4 * i, u);
     }
     FacePoint<T> f;
     if (is_fp) {
-        load_face_point<N1>(a, e, edge, fp, f);
+        const T* Tin = after_wait(a.Tin);
+        load_own_face<N1>(a, Tin, e, edge, fp, f);
+        load_neighbour_face<N1>(a, Tin, fp, f);
         T d[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) d[v] = (f.r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (f.qn[v] - f.qo[v]);
-        store4(sDU + el * DS + k * 4, d);
+        store4(sDU + el * DP + face_slot<P, T>(fl.dir, fl.side, fl.line), d);
     }
     __syncthreads();
     if (is_sp) {
         T Qx[4], Qy[4];
-        corrected_gradient_tr<N1, RS, VS>(sU + el * FS, sUt + el * FS, sDU + el * DS, sOps, i, j, ji, Qx, Qy);
-        T* sq = sQ + el * QS + j * RS + i;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) { sq[v * VS] = Qx[v]; sq[(4 + v) * VS] = Qy[v]; }
+        corrected_gradient<P>(sU + el * FP, sDU + el * DP, sOps, i, j, ji, Qx, Qy);
+        store4(sQx + el * FP + j * RP + 4 * i, Qx);
+        store4(sQy + el * FP + j * RP + 4 * i, Qy);
     }
     __syncthreads();
     if (is_fp) {
         T t[8];
-        trace_point<N1, RS, VS>(sQ + el * QS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
-        trace_point<N1, RS, VS>(sQ + el * QS + 4 * VS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge,
-                                fp, t + 4);
-        if (a.GQ) gstore8(a.GQ + (e * NFT + k) * 8, t);
+        state_trace<P>(sQx + el * FP, sOps, fl, t);
+        state_trace<P>(sQy + el * FP, sOps, fl, t + 4);
+        if (a.GQ) gstore8(a.GQ + (e * NFT + kf) * 8, t);
         if (a.FVout) {
             T Ua[4], fv[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) Ua[v] = T(0.5) * (f.qo[v] + f.qn[v]);
             viscous_share(a, f.r, f.nx, f.ny, Ua, t, fv);
-            gstore4(a.FVout + (e * NFT + k) * 4, fv);
+            gstore4(a.FVout + (e * NFT + kf) * 4, fv);
         }
     }
 }
@@ -383,16 +335,17 @@ k_ns_grad_lines(const StageArgsT<T> a) {
     // end points
     T dA[4], dB[4];
     T UaA[4], UaB[4];
+    const T* Tin = after_wait(a.Tin);
     if (valid) {
 #pragma unroll
         for (int s2 = 0; s2 < 2; ++s2) {
             const int ed = s2 ? eB : eA, fp = s2 ? fB : fA;
             const EdgeRec r = a.edges[e * 4 + ed];
             T qo[4], qn[4];
-            load4_nc(a.Tin + (e * NFT + ed * N1 + fp) * 4, qo);
+            load4_nc(Tin + (e * NFT + ed * N1 + fp) * 4, qo);
 #pragma unroll
             for (int v = 0; v < 4; ++v) qn[v] = qo[v];
-            if (!(r.flags & kEdgeOrphan)) load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
+            if (!(r.flags & kEdgeOrphan)) load4_nc(Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
             T* d = s2 ? dB : dA;
             T* m = s2 ? UaB : UaA;
 #pragma unroll
@@ -505,19 +458,17 @@ __global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS, NSMinBlock
 k_ns_stage(const StageArgsT<T> a) {
     using S = Shape<P, EbDiv<T>::value>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = Tiles<P, T>::FS, DS = Tiles<P, T>::DS;
-    __shared__ T sOps[S::NOPS];
-    // From P4 up the G~ tile is held transposed ([var][xi][eta]), so its
-    // eta-lines (divergence, traces of edges 0 and 2) are row loads
-    constexpr bool kTrG = P >= 4;
-    __shared__ __align__(16) T sF[EB * FS];
-    __shared__ __align__(16) T sG[EB * FS];
-    __shared__ __align__(16) T sD[EB * DS];   // face jumps of U, then flux differences
-    __shared__ __align__(16) T sU[EB * FS];   // stage state, then the new state
+    using Op = OpTable<P + 1, T>;
+    constexpr int RP = Tiles<P, T>::RP, FP = Tiles<P, T>::FP, DP = Tiles<P, T>::DP;
+    __shared__ __align__(16) Weight<T> sOps[Op::N];
+    __shared__ __align__(16) T sF[EB * FP];
+    __shared__ __align__(16) T sG[EB * FP];
+    __shared__ __align__(16) T sD[EB * DP];   // face jumps of U, then flux differences
+    __shared__ __align__(16) T sU[EB * FP];   // stage state, then the new state
     __shared__ double sRed[32];
 
     const int tid = threadIdx.x;
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    Op::fill(sOps, a.ops);
     pdl_launch_dependents();
     pdl_wait();   // the viscous shares come from the gradient launch, the state from the previous stage
     const int el = tid / TPE, k = tid - el * TPE;
@@ -525,69 +476,101 @@ k_ns_stage(const StageArgsT<T> a) {
     const long long e = block_element(a, EB, el, valid);
     const bool is_sp = valid && k < NSP, is_fp = valid && k < NFT;
     const T g = T(a.gamma);
-    const int edge = k / N1, fp = k - edge * N1;
-    const int i = k % N1, j = k / N1;
+    const FaceLane fl = lane_face<N1>(k);
+    const int edge = fl.edge, fp = fl.fp, kf = edge * N1 + fp;
+    int i, j;
+    lane_point<N1>(k, i, j);
+    const int ks = j * N1 + i;
 
     // ---- A1: loads, face jumps, stage state into shared memory; the common
     // flux of the flux points, which needs nothing else (a thread carries its
     // four values, not the traces they came from, through the volume phase)
-    FacePoint<T> f;
     constexpr bool kRef = UsesRef<T>::value;
     T ue[4] = {T(0), T(0), T(0), T(0)};   // reference state (mixed form)
-    if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
     T u[4], ji[4], Jd = T(1);
     T Fd[4] = {T(0), T(0), T(0), T(0)};
-    if (is_sp) {
-        const long long idx = e * NSP + k;
-        double ud[4];
+    const T* Tin = after_wait(a.Tin);
+    const T* FV = after_wait(a.FV);
+    FacePoint<T> f;
+    f.r = EdgeRec{-1, 0, kEdgeOrphan, 0};
+    T fo[4], fn[4] = {T(0), T(0), T(0), T(0)};
+    double ud[4];
+    auto load_point = [&] {
+        const long long idx = e * NSP + ks;
         stage_state(a, idx, ud, u);
-        load4_nc(a.Jinv + idx * 4, ji);
+        load4_x(a.Jinv + idx * 4, ji);
         Jd = ldg_any(a.J + idx);
-        if ((k & 3) == 0 && a.stage >= 2) prefetch_l2(a.U0 + idx * 4);
-        T* su = sU + el * FS + j * RS + i;
+        if ((ks & 3) == 0 && a.stage >= 2) prefetch_l2(a.U0 + idx * 4);
+    };
+    auto store_point = [&] {
         T w[4];
         if constexpr (kRef) state_minus_ref(ud, ue, w);
         else {
 #pragma unroll
             for (int v = 0; v < 4; ++v) w[v] = u[v];
         }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) su[v * VS] = w[v];
+        store4(sU + el * FP + j * RP + 4 * i, w);
+    };
+    // FP32 issues every load before the first use, the edge record first (the
+    // neighbour's rows hang on it): -6 % per step at 256 x 256, P3.  In FP64
+    // that is 56 registers of data in flight and was slower; there the
+    // solution point goes first and the face's loads are the compiler's to place.
+    if constexpr (sizeof(T) == 4) {
+        if (is_fp) {
+            load_own_face<N1>(a, Tin, e, edge, fp, f);
+            load4_now(FV + (e * NFT + kf) * 4, fo);
+        }
+        if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
+        if (is_sp) load_point();
+        if (is_fp) {
+            load_neighbour_face<N1>(a, Tin, fp, f);
+            if (has_neighbour_gradient(f.r))
+                load4_now(FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
+        }
+        if (is_sp) store_point();
+    } else {
+        if (is_sp) {
+            load_point();
+            store_point();
+        }
+        if (is_fp) {
+            load_own_face<N1>(a, Tin, e, edge, fp, f);
+            load_neighbour_face<N1>(a, Tin, fp, f);
+            load4_nc(FV + (e * NFT + kf) * 4, fo);
+            if (has_neighbour_gradient(f.r))
+                load4_nc(FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
+        }
     }
+    const bool face = is_fp && !(f.r.flags & kEdgeOrphan);
     if (is_fp) {
-        T fo[4], fn[4] = {T(0), T(0), T(0), T(0)};
-        load_face_point<N1>(a, e, edge, fp, f);
-        load4_nc(a.FV + (e * NFT + k) * 4, fo);
-        if (has_neighbour_gradient(f.r))
-            load4_nc(a.FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
         T d[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) d[v] = (f.r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (f.qn[v] - f.qo[v]);
-        store4(sD + el * DS + k * 4, d);
-        if (!(f.r.flags & kEdgeOrphan)) {
-            // evaluated from the left element's side on both sides
-            const bool right = (f.r.flags & kEdgeRight) != 0;
-            T UL[4], UR[4], Fc[4];
+        for (int v = 0; v < 4; ++v) d[v] = face ? T(0.5) * (f.qn[v] - f.qo[v]) : T(0);
+        store4(sD + el * DP + face_slot<P, T>(fl.dir, fl.side, fl.line), d);
+    }
+    if (face) {
+        // evaluated from the left element's side on both sides
+        const bool right = (f.r.flags & kEdgeRight) != 0;
+        T UL[4], UR[4], Fc[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) { UL[v] = right ? f.qn[v] : f.qo[v]; UR[v] = right ? f.qo[v] : f.qn[v]; }
-            riemann<RIEM>(UL, UR, f.nx, f.ny, g, Fc);
-            if constexpr (kRef) {
-                T Fe[4];
-                ref_flux_n(ue, g, f.nx, f.ny, Fe);
+        for (int v = 0; v < 4; ++v) { UL[v] = right ? f.qn[v] : f.qo[v]; UR[v] = right ? f.qo[v] : f.qn[v]; }
+        riemann<RIEM>(UL, UR, f.nx, f.ny, g, Fc);
+        if constexpr (kRef) {
+            T Fe[4];
+            ref_flux_n(ue, g, f.nx, f.ny, Fe);
 #pragma unroll
-                for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
-            }
-            const T ss = right ? T(-0.5) * f.len : T(0.5) * f.len;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) Fd[v] = ss * (Fc[v] - (fo[v] + fn[v]));
+            for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
         }
+        const T ss = right ? T(-0.5) * f.len : T(0.5) * f.len;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Fd[v] = ss * (Fc[v] - (fo[v] + fn[v]));
     }
     __syncthreads();
 
     // ---- A2: gradient, total transformed fluxes
     if (is_sp) {
         T Qx[4], Qy[4], Fv[4], Gv[4];
-        corrected_gradient<N1, RS, VS>(sU + el * FS, sD + el * DS, sOps, i, j, ji, Qx, Qy);
+        corrected_gradient<P>(sU + el * FP, sD + el * DP, sOps, i, j, ji, Qx, Qy);
         // one reciprocal density for the viscous and the Euler flux
         const T ir = rcp_any(u[0]);
         viscous_flux_f(u, ir, Qx, Qy, g, inv_reynolds(a), T(a.kfac), Fv, Gv);
@@ -601,77 +584,28 @@ k_ns_stage(const StageArgsT<T> a) {
         }
 #pragma unroll
         for (int v = 0; v < 4; ++v) { F[v] -= Fv[v]; G[v] -= Gv[v]; }
-        T* fo = sF + el * FS + j * RS + i;
-        T* ho = sG + el * FS + (kTrG ? i * RS + j : j * RS + i);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            fo[v * VS] = Jd * (ji[0] * F[v] + ji[1] * G[v]);
-            ho[v * VS] = Jd * (ji[2] * F[v] + ji[3] * G[v]);
-        }
+        store_fluxes<P>(sF + el * FP, sG + el * FP, i, j, Jd, ji, F, G);
     }
     __syncthreads();   // face jumps and the stage state in shared memory are dead now
 
     // ---- B: flux differences at the faces
     if (is_fp) {
-        if (!(f.r.flags & kEdgeOrphan)) {
-            const bool along_eta = (edge == 0 || edge == 2);
-            T Fn[4];
-            if constexpr (kTrG)
-                trace_row<N1, RS, VS>((along_eta ? sG : sF) + el * FS,
-                                      (edge == 0 || edge == 3) ? sOps + N1 * N1 : sOps + N1 * N1 + N1,
-                                      (edge >= 2) ? (N1 - 1 - fp) : fp, Fn);
-            else
-                trace_point<N1, RS, VS>((along_eta ? sG : sF) + el * FS, sOps + N1 * N1,
-                                        sOps + N1 * N1 + N1, edge, fp, Fn);
-            const T sgn = (edge == 0 || edge == 3) ? T(-1) : T(1);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) Fd[v] -= sgn * Fn[v];
-        }
-        store4(sD + el * DS + k * 4, Fd);
+        if (face) flux_difference<P>((fl.dir ? sF : sG) + el * FP, sOps, fl, Fd);
+        store4(sD + el * DP + face_slot<P, T>(fl.dir, fl.side, fl.line), Fd);
     }
     __syncthreads();
 
     // ---- C: divergence, VCJH correction, 1/J, stage update
     double rsq = 0.0;
     if (is_sp) {
-        const long long idx = e * NSP + k;
+        const long long idx = e * NSP + ks;
         double u0[4];
         if (a.stage >= 2) gload4(a.U0 + idx * 4, u0);
-        T Di[N1], Dj[N1];
-#pragma unroll
-        for (int m = 0; m < N1; ++m) { Di[m] = sOps[i * N1 + m]; Dj[m] = sOps[j * N1 + m]; }
-        const T* gL = sOps + N1 * N1 + 2 * N1;
-        const T* gR = gL + N1;
-        const T gRi = gR[i], gLi = gL[i], gRj = gR[j], gLj = gL[j];
-        const T* fo = sF + el * FS;
-        const T* ho = sG + el * FS;
-        const T* d = sD + el * DS;
-        T c1[4], c3[4], c2[4], c0[4];
-        load4(d + (1 * N1 + j) * 4, c1);
-        load4(d + (3 * N1 + (N1 - 1 - j)) * 4, c3);
-        load4(d + (2 * N1 + (N1 - 1 - i)) * 4, c2);
-        load4(d + (0 * N1 + i) * 4, c0);
         const T iJ = rcp_any(Jd);
         T res[4];
+        divergence<P>(sF + el * FP, sG + el * FP, sD + el * DP, sOps, i, j, res);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            T fr[N1];
-            load_row<N1>(fo + v * VS + j * RS, fr);
-            T div = T(0);
-#pragma unroll
-            for (int m = 0; m < N1; ++m) div = fma_any(Di[m], fr[m], div);
-            if constexpr (kTrG) {
-                T gc[N1];
-                load_row<N1>(ho + v * VS + i * RS, gc);
-#pragma unroll
-                for (int m = 0; m < N1; ++m) div = fma_any(Dj[m], gc[m], div);
-            } else {
-#pragma unroll
-                for (int m = 0; m < N1; ++m) div = fma_any(Dj[m], ho[v * VS + m * RS + i], div);
-            }
-            const T corr = gRi * c1[v] - gLi * c3[v] + gRj * c2[v] - gLj * c0[v];
-            res[v] = -(div + corr) * iJ;
-        }
+        for (int v = 0; v < 4; ++v) res[v] = -res[v] * iJ;
         if (a.stage == 0) {
             store_residual(a, idx, res, rsq);
         } else {
@@ -685,15 +619,13 @@ k_ns_stage(const StageArgsT<T> a) {
             double uo[4];
             rk_update(a.stage, *a.dt, us, u0, res, uo);
             gstore4(a.Uout + idx * 4, uo);
-            T* su = sU + el * FS + j * RS + i;
             T un[4];
             if constexpr (kRef) state_minus_ref(uo, ue, un);
             else {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) un[v] = T(uo[v]);
             }
-#pragma unroll
-            for (int v = 0; v < 4; ++v) su[v * VS] = un[v];
+            store4(sU + el * FP + j * RP + 4 * i, un);
             if (a.stage == 3) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) rsq += double(res[v]) * double(res[v]);
@@ -710,12 +642,12 @@ k_ns_stage(const StageArgsT<T> a) {
     // ---- D: traces of the new state
     if (is_fp) {
         T t[4];
-        trace_point<N1, RS, VS>(sU + el * FS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
+        state_trace<P>(sU + el * FP, sOps, fl, t);
         if constexpr (kRef) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) t[v] += ue[v];
         }
-        gstore4(a.Tout + (e * NFT + k) * 4, t);
+        gstore4(a.Tout + (e * NFT + kf) * 4, t);
         if (boundary_condition_edge(f.r)) store_ghost<N1>(a, f.r, f.nx, f.ny, fp, t);
     }
 }

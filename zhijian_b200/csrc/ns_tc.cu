@@ -60,14 +60,14 @@ template <int P>
 struct TcSmem {
     using C = TcShape<P>;
     using S = Shape<P>;
-    static constexpr int FS = Tiles<P, float>::FS, DS = Tiles<P, float>::DS;
+    static constexpr int FP = Tiles<P, float>::FP, DP = Tiles<P, float>::DP;
     static constexpr size_t A_OFF = 0;
     static constexpr size_t B_OFF = A_OFF + 2 * C::A_TERM;
     static constexpr size_t R_OFF = B_OFF + 2 * C::B_TERM;
     static constexpr size_t OPS_OFF = R_OFF + sizeof(float) * C::M * C::RS_;
-    static constexpr size_t U_OFF = OPS_OFF + sizeof(float) * ((S::NOPS + 3) & ~3);
-    static constexpr size_t D_OFF = U_OFF + sizeof(float) * C::EB * FS;
-    static constexpr size_t RED_OFF = (D_OFF + sizeof(float) * C::EB * DS + 7) & ~size_t(7);
+    static constexpr size_t U_OFF = OPS_OFF + ((sizeof(Weight<float>) * OpTable<P + 1, float>::N + 15) & ~size_t(15));
+    static constexpr size_t D_OFF = U_OFF + sizeof(float) * C::EB * FP;
+    static constexpr size_t RED_OFF = (D_OFF + sizeof(float) * C::EB * DP + 7) & ~size_t(7);
     static constexpr size_t BAR_OFF = RED_OFF + sizeof(double) * 32;
     static constexpr size_t SLOT_OFF = BAR_OFF + 2 * sizeof(uint64_t);
     static constexpr size_t BYTES = SLOT_OFF + 16;
@@ -96,12 +96,13 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
     using C = TcShape<P>;
     using L = TcSmem<P>;
     constexpr int N1 = C::N1, NSP = C::NSP, NFT = C::NFT, TPE = C::TPE, EB = C::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = L::FS, DS = L::DS;
+    using Op = OpTable<P + 1, float>;
+    constexpr int RP = Tiles<P, float>::RP, FP = L::FP, DP = L::DP;
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char* sA = smem + L::A_OFF;
     unsigned char* sB = smem + L::B_OFF;
     float* sR = reinterpret_cast<float*>(smem + L::R_OFF);
-    float* sOps = reinterpret_cast<float*>(smem + L::OPS_OFF);
+    Weight<float>* sOps = reinterpret_cast<Weight<float>*>(smem + L::OPS_OFF);
     float* sU = reinterpret_cast<float*>(smem + L::U_OFF);
     float* sD = reinterpret_cast<float*>(smem + L::D_OFF);
     double* sRed = reinterpret_cast<double*>(smem + L::RED_OFF);
@@ -120,7 +121,7 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
     // stale shared memory would not be)
     for (int t = tid; t < 2 * C::B_TERM / 16; t += blockDim.x)
         reinterpret_cast<uint4*>(sB)[t] = make_uint4(0u, 0u, 0u, 0u);
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    Op::fill(sOps, a.ops);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
@@ -147,7 +148,9 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
     f.r = EdgeRec{-1, 0, kEdgeOrphan, 0};
     float fv[4] = {0.f, 0.f, 0.f, 0.f};   // common normal viscous flux: both sides' shares
     if (is_fp) {
-        load_face_point<N1>(a, e, edge, fp, f);
+        const float* Tin = after_wait(a.Tin);
+        load_own_face<N1>(a, Tin, e, edge, fp, f);
+        load_neighbour_face<N1>(a, Tin, fp, f);
         load4_nc(a.FV + (e * NFT + k) * 4, fv);
         if (has_neighbour_gradient(f.r)) {
             float fn[4];
@@ -158,7 +161,8 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
         float d[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) d[v] = (f.r.flags & kEdgeOrphan) ? 0.f : 0.5f * (f.qn[v] - f.qo[v]);
-        store4(sD + el * DS + k * 4, d);
+        const int dir = edge & 1, side = (edge == 1 || edge == 2);
+        store4(sD + el * DP + face_slot<P, float>(dir, side, (dir == side) ? fp : N1 - 1 - fp), d);
     }
     float ue[4] = {0.f, 0.f, 0.f, 0.f};   // the element's reference state
     if (valid) load_state(a.U + e * NSP * 4, ue);
@@ -172,16 +176,14 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
         if ((k & 3) == 0 && a.stage >= 2) prefetch_l2(a.U0 + idx * 4);
         float w[4];
         state_minus_ref(ud, ue, w);
-        float* su = sU + el * FS + j * RS + i;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) su[v * VS] = w[v];
+        store4(sU + el * FP + j * RP + 4 * i, w);
     }
     __syncthreads();
 
     // ---- A2: gradient, total transformed fluxes as the BF16 pairs of B
     if (is_sp) {
         float Qx[4], Qy[4], Fv[4], Gv[4];
-        corrected_gradient<N1, RS, VS>(sU + el * FS, sD + el * DS, sOps, i, j, ji, Qx, Qy);
+        corrected_gradient<P>(sU + el * FP, sD + el * DP, sOps, i, j, ji, Qx, Qy);
         const float ir = rcp_any(u[0]);
         viscous_flux_f(u, ir, Qx, Qy, g, inv_reynolds(a), float(a.kfac), Fv, Gv);
         float F[4], G[4], Fe[4], Ge[4];
@@ -277,7 +279,8 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
 #pragma unroll
             for (int v = 0; v < 4; ++v) Fd[v] = ss * Fc[v] - sgn * Fn[v];
         }
-        store4(sD + el * DS + k * 4, Fd);
+        const int dir = edge & 1, side = (edge == 1 || edge == 2);
+        store4(sD + el * DP + face_slot<P, float>(dir, side, (dir == side) ? fp : N1 - 1 - fp), Fd);
     }
     __syncthreads();
 
@@ -287,24 +290,11 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
         const long long idx = e * NSP + k;
         double u0[4];
         if (a.stage >= 2) gload4(a.U0 + idx * 4, u0);
-        const float* gL = sOps + N1 * N1 + 2 * N1;
-        const float* gR = gL + N1;
-        const float gRi = gR[i], gLi = gL[i], gRj = gR[j], gLj = gL[j];
-        const float* d = sD + el * DS;
-        float c1[4], c3[4], c2[4], c0[4];
-        load4(d + (1 * N1 + j) * 4, c1);
-        load4(d + (3 * N1 + (N1 - 1 - j)) * 4, c3);
-        load4(d + (2 * N1 + (N1 - 1 - i)) * 4, c2);
-        load4(d + (0 * N1 + i) * 4, c0);
-        const float4 dv = *reinterpret_cast<const float4*>(sR + k * C::RS_ + el * 4);
-        const float div[4] = {dv.x, dv.y, dv.z, dv.w};
         const float iJ = rcp_any(Jd);
         float res[4];
+        v4_get(correction<P>(sD + el * DP, sOps, i, j, v4_load(sR + k * C::RS_ + el * 4)), res);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const float corr = gRi * c1[v] - gLi * c3[v] + gRj * c2[v] - gLj * c0[v];
-            res[v] = -(div[v] + corr) * iJ;
-        }
+        for (int v = 0; v < 4; ++v) res[v] = -res[v] * iJ;
         if (a.stage == 0) {
             store_residual(a, idx, res, rsq);
         } else {
@@ -315,9 +305,7 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
             gstore4(a.Uout + idx * 4, uo);
             float un[4];
             state_minus_ref(uo, ue, un);
-            float* su = sU + el * FS + j * RS + i;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) su[v * VS] = un[v];
+            store4(sU + el * FP + j * RP + 4 * i, un);
             if (a.stage == 3) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) rsq += double(res[v]) * double(res[v]);
@@ -333,7 +321,8 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
     // ---- D: traces of the new state
     if (a.stage != 0 && is_fp) {
         float t[4];
-        trace_point<N1, RS, VS>(sU + el * FS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
+        const int dir = edge & 1, side = (edge == 1 || edge == 2);
+        state_trace<P>(sU + el * FP, sOps, FaceLane{dir, (dir == side) ? fp : N1 - 1 - fp, side, edge, fp}, t);
 #pragma unroll
         for (int v = 0; v < 4; ++v) t[v] += ue[v];
         gstore4(a.Tout + (e * NFT + k) * 4, t);
@@ -391,7 +380,7 @@ cudaError_t ns_stage_tc_p(int riemann, const StageArgs32& a, const CUtensorMap& 
 // Host image of A for order P: [term hi, lo][chunk K/8][row M][8] BF16, rows
 // 0..n_sp-1 the divergence of solution point k = j n1 + i (D1[i][m] at
 // K = j n1 + m on F~, D1[j][m] at K = n_sp + m n1 + i on G~), rows
-// n_sp + edge n1 + fp the edge traces in trace_point's order (edge 0: Lm on
+// n_sp + edge n1 + fp the edge traces by edge and point (edge 0: Lm on
 // G~ column fp; 1: Lp on F~ row fp; 2: Lp on G~ column n1-1-fp; 3: Lm on F~
 // row n1-1-fp).
 template <int P>

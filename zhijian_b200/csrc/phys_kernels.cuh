@@ -41,24 +41,20 @@ namespace {
 using namespace dev;
 using namespace phys;
 
-// Per-element strides of the shared tiles.  Double tiles (two 4-byte banks
-// per value): [var][row][col] fields at 6 mod 16 doubles and the
-// [flux point][var] tile at 2 mod 16 (Shape).  Float tiles: every stride a
-// multiple of 4 floats (16-byte rows) and congruent mod 32 to the threads per
-// element (rounded up to a multiple of 4), so the elements that share a warp
-// start on disjoint banks.
+// Strides of the shared tiles, in values.  A field tile holds point (i, j) at
+// j * RP + 4 i with its four variables; the rows are padded so that the points
+// of a row and those of a column fall on distinct banks, the elements by RP's
+// padding once more.  The flux-point tile is [dir][side][line][var]: the four
+// loads of a solution point (its lines' ends) spread over the banks too.
 template <int P, typename T>
 struct Tiles {
     using S = Shape<P, EbDiv<T>::value>;
-    static constexpr int pad32(int base) {
-        return base + ((((S::TPE + 3) & ~3) % 32) - base % 32 + 64) % 32;
-    }
-    static constexpr bool kD = sizeof(T) == 8;
-    static constexpr int FS = kD ? S::FS : pad32(4 * S::VS);         // one field of 4 vars
-    static constexpr int DS = kD ? S::DS : pad32(4 * S::NFT);        // flux-point tile
-    static constexpr int QS = kD ? 8 * S::VS + (6 - (8 * S::VS) % 16 + 16) % 16
-                                 : pad32(8 * S::VS);                 // gradient field
-    static_assert(kD || (FS % 4 == 0 && DS % 4 == 0 && QS % 4 == 0), "16-byte float rows");
+    static constexpr int N1 = S::N1;
+    static constexpr int PAD = sizeof(T) == 4 ? 4 : (sizeof(T) == 8 ? 2 : 1);   // 16 bytes
+    static constexpr int RP = 4 * N1 + PAD;
+    static constexpr int FP = N1 * RP;
+    static constexpr int DB = 4 * N1 + (sizeof(T) == 4 ? 0 : PAD);              // one (dir, side) block
+    static constexpr int DP = 4 * DB + PAD * (sizeof(T) == 4 ? 4 : 1);
 };
 
 // Element of thread group el of this CTA: through the element list of a
@@ -116,7 +112,7 @@ __device__ __forceinline__ void store_ghost(const StageArgsT<T>& a, const EdgeRe
 template <typename T>
 __device__ __forceinline__ void load_state(const double* p, T* u) {
     double d[4];
-    gload4(p, d);
+    load4_now(p, d);
 #pragma unroll
     for (int v = 0; v < 4; ++v) u[v] = T(d[v]);
 }
@@ -230,21 +226,100 @@ template <> struct PhysMinBlocks<double> { static constexpr int value = ZJ_PHYS_
 template <> struct PhysMinBlocks<float> { static constexpr int value = ZJ_PHYS32_MIN_BLOCKS * kCtaScale; };
 template <> struct PhysMinBlocks<Dual> { static constexpr int value = 1; };
 
+// Offset of a flux point in the [dir][side][line][var] tile.
+template <int P, typename T>
+__device__ __forceinline__ int face_slot(int dir, int side, int line) {
+    return (dir * 2 + side) * Tiles<P, T>::DB + line * 4;
+}
+
+// Transformed fluxes F~ = J (xi_x F + xi_y G), G~ = J (eta_x F + eta_y G) of
+// point (i, j) into the tiles.
+template <int P, typename T>
+__device__ __forceinline__ void store_fluxes(T* tF, T* tG, int i, int j, T Jd, const T* ji, const T* F,
+                                             const T* G) {
+    constexpr int RP = Tiles<P, T>::RP;
+    T ft[4], gt[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        ft[v] = Jd * (ji[0] * F[v] + ji[1] * G[v]);
+        gt[v] = Jd * (ji[2] * F[v] + ji[3] * G[v]);
+    }
+    store4(tF + j * RP + 4 * i, ft);
+    store4(tG + j * RP + 4 * i, gt);
+}
+
+// The line of a tile that a flux point ends: first point and stride.
+template <int P, typename T>
+__device__ __forceinline__ const T* line_of(const T* tile, const FaceLane& f, int& stride) {
+    constexpr int RP = Tiles<P, T>::RP;
+    stride = f.dir ? 4 : RP;
+    return tile + f.line * (f.dir ? RP : 4);
+}
+
+// Fd minus the outward extrapolated transformed flux of a flux point (tile:
+// F~ for xi-lines, G~ for eta-lines; outward is -F~ at -1, +F~ at +1).
+template <int P, typename T>
+__device__ __forceinline__ void flux_difference(const T* tile, const Weight<T>* ops, const FaceLane& f, T* Fd) {
+    using Op = OpTable<P + 1, T>;
+    constexpr int N1 = P + 1;
+    int stride;
+    const T* p = line_of<P>(tile, f, stride);
+    Weight<T> w[N1];
+    load_weights<N1>(ops + (f.side ? Op::NLP : Op::LM), w);
+    v4_get(line_dot<N1>(w, p, stride, v4(Fd)), Fd);
+}
+
+// Trace of a state tile at a flux point.
+template <int P, typename T>
+__device__ __forceinline__ void state_trace(const T* tile, const Weight<T>* ops, const FaceLane& f, T* t) {
+    using Op = OpTable<P + 1, T>;
+    constexpr int N1 = P + 1;
+    int stride;
+    const T* p = line_of<P>(tile, f, stride);
+    Weight<T> w[N1];
+    load_weights<N1>(ops + (f.side ? Op::LP : Op::LM), w);
+    v4_get(line_dot<N1>(w, p, stride, v4_zero<T>()), t);
+}
+
+// acc + the VCJH corrections with the flux differences d at point (i, j).
+template <int P, typename T>
+__device__ __forceinline__ V4<T> correction(const T* d, const Weight<T>* ops, int i, int j, V4<T> acc) {
+    using Op = OpTable<P + 1, T>;
+    acc = v4_fma(ops[Op::GR + i], v4_load(d + face_slot<P, T>(1, 1, j)), acc);
+    acc = v4_fma(ops[Op::NGL + i], v4_load(d + face_slot<P, T>(1, 0, j)), acc);
+    acc = v4_fma(ops[Op::GR + j], v4_load(d + face_slot<P, T>(0, 1, i)), acc);
+    return v4_fma(ops[Op::NGL + j], v4_load(d + face_slot<P, T>(0, 0, i)), acc);
+}
+
+// D_xi F~ + D_eta G~ + the corrections at point (i, j).
+template <int P, typename T>
+__device__ __forceinline__ void divergence(const T* tF, const T* tG, const T* d, const Weight<T>* ops, int i,
+                                           int j, T* out) {
+    constexpr int N1 = P + 1, RP = Tiles<P, T>::RP;
+    Weight<T> w[N1];
+    load_weights<N1>(ops + i * N1, w);
+    V4<T> acc = line_dot<N1>(w, tF + j * RP, 4, v4_zero<T>());
+    load_weights<N1>(ops + j * N1, w);
+    acc = line_dot<N1>(w, tG + 4 * i, RP, acc);
+    v4_get(correction<P>(d, ops, i, j, acc), out);
+}
+
 template <int P, int RIEM, typename T>
 __global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS, PhysMinBlocks<T>::value)
 k_phys_stage(const StageArgsT<T> a) {
     using S = Shape<P, EbDiv<T>::value>;
+    using Op = OpTable<P + 1, T>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = Tiles<P, T>::FS, DS = Tiles<P, T>::DS;
-    __shared__ T sOps[S::NOPS];
-    __shared__ __align__(16) T sF[EB * FS];
-    __shared__ __align__(16) T sG[EB * FS];
-    __shared__ __align__(16) T sD[EB * DS];
-    __shared__ __align__(16) T sU[EB * FS];
+    constexpr int RP = Tiles<P, T>::RP, FP = Tiles<P, T>::FP, DP = Tiles<P, T>::DP;
+    __shared__ __align__(16) Weight<T> sOps[Op::N];
+    __shared__ __align__(16) T sF[EB * FP];
+    __shared__ __align__(16) T sG[EB * FP];
+    __shared__ __align__(16) T sD[EB * DP];
+    __shared__ __align__(16) T sU[EB * FP];
     __shared__ double sRed[32];
 
     const int tid = threadIdx.x;
-    for (int i = tid; i < S::NOPS; i += blockDim.x) sOps[i] = a.ops[i];
+    Op::fill(sOps, a.ops);
     pdl_launch_dependents();
     pdl_wait();   // the state and traces come from the previous stage
 
@@ -254,29 +329,38 @@ k_phys_stage(const StageArgsT<T> a) {
     const bool is_sp = valid && k < NSP;
     const bool is_fp = valid && k < NFT;
     const T g = T(a.gamma);
-    const int edge = k / N1, fp = k - edge * N1;
-    const int i = k % N1, j = k / N1;
+    const FaceLane fl = lane_face<N1>(k);
+    const int edge = fl.edge, fp = fl.fp, kf = edge * N1 + fp;
+    int i, j;
+    lane_point<N1>(k, i, j);
+    const int ks = j * N1 + i;
 
-    // ---- A: loads; transformed fluxes into shared memory
+    // ---- A: loads; transformed fluxes into shared memory; common fluxes
     constexpr bool kRef = UsesRef<T>::value;
-    EdgeRec r{-1, 0, kEdgeOrphan, 0};
-    T nr[3] = {T(0), T(0), T(0)};
-    T qo[4], qn[4] = {T(0), T(0), T(0), T(0)}, u[4], Jd = T(1);
+    // (loads first, the edge record ahead of all: the neighbour's row hangs on it)
+    T u[4], Jd = T(1);
+    T Fd[4] = {T(0), T(0), T(0), T(0)};
     T ue[4] = {T(0), T(0), T(0), T(0)};   // reference state (mixed form)
-    if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
+    T nr[3], qo[4], qn[4], ji[4];
+    double ud[4];
+    EdgeRec r{-1, 0, kEdgeOrphan, 0};
     if (is_fp) {
         r = a.edges[e * 4 + edge];
+        load4_now(a.Tin + (e * NFT + kf) * 4, qo);
         load_normal(normal_rec<N1>(a, e, edge, fp), nr);
-        load4_nc(a.Tin + (e * NFT + k) * 4, qo);
     }
+    if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
     if (is_sp) {
-        const long long idx = e * NSP + k;
-        double ud[4];
+        const long long idx = e * NSP + ks;
         stage_state(a, idx, ud, u);
-        T ji[4];
-        load4_nc(a.Jinv + idx * 4, ji);
+        load4_now(a.Jinv + idx * 4, ji);
         Jd = ldg_any(a.J + idx);
-        if ((k & 3) == 0 && a.stage >= 2) prefetch_l2(a.U0 + idx * 4);
+        if ((ks & 3) == 0 && a.stage >= 2) prefetch_l2(a.U0 + idx * 4);
+    }
+    const bool face = is_fp && !(r.flags & kEdgeOrphan);
+    const bool bc_face = is_fp && boundary_condition_edge(r);
+    if (face) load4_now(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
+    if (is_sp) {
         T F[4], G[4];
         euler_flux(u, g, F, G);
         if constexpr (kRef) {
@@ -285,87 +369,48 @@ k_phys_stage(const StageArgsT<T> a) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) { F[v] -= Fe[v]; G[v] -= Ge[v]; }
         }
-        T* f = sF + el * FS + j * RS + i;
-        T* h = sG + el * FS + j * RS + i;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            f[v * VS] = Jd * (ji[0] * F[v] + ji[1] * G[v]);
-            h[v * VS] = Jd * (ji[2] * F[v] + ji[3] * G[v]);
-        }
+        store_fluxes<P>(sF + el * FP, sG + el * FP, i, j, Jd, ji, F, G);
     }
-    // The neighbour's point that coincides with this one: both elements run
-    // their shared edge counter-clockwise.
-    if (is_fp && !(r.flags & kEdgeOrphan))
-        load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
+    // The common flux of a flux point, from the own and the neighbour's point
+    // that coincides with it (both elements run their shared edge
+    // counter-clockwise); evaluated from the left element's side on both
+    // sides of a face (bit-identical on both).
+    if (face) {
+        const bool right = (r.flags & kEdgeRight) != 0;
+        T UL[4], UR[4], Fc[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) { UL[v] = right ? qn[v] : qo[v]; UR[v] = right ? qo[v] : qn[v]; }
+        riemann<RIEM>(UL, UR, nr[0], nr[1], g, Fc);
+        if constexpr (kRef) {
+            T Fe[4];
+            ref_flux_n(ue, g, nr[0], nr[1], Fe);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
+        }
+        const T ss = right ? T(-0.5) * nr[2] : T(0.5) * nr[2];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Fd[v] = ss * Fc[v];
+    }
     __syncthreads();   // sOps, sF, sG ready
 
-    // ---- B: interface terms.  The common flux is evaluated from the left
-    // element's side on both sides of a face (bit-identical on both).
+    // ---- B: flux differences at the faces
     if (is_fp) {
-        T Fd[4] = {T(0), T(0), T(0), T(0)};
-        if (!(r.flags & kEdgeOrphan)) {
-            const T nx = nr[0], ny = nr[1], s = T(0.5) * nr[2];
-            const bool right = (r.flags & kEdgeRight) != 0;
-            T UL[4], UR[4], Fc[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) { UL[v] = right ? qn[v] : qo[v]; UR[v] = right ? qo[v] : qn[v]; }
-            riemann<RIEM>(UL, UR, nx, ny, g, Fc);
-            if constexpr (kRef) {
-                T Fe[4];
-                ref_flux_n(ue, g, nx, ny, Fe);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
-            }
-            const T ss = right ? -s : s;
-            // Extrapolated transformed flux along this element's outward
-            // reference normal: +F~ on edge 1, -F~ on edge 3, -G~ on edge 0,
-            // +G~ on edge 2.
-            const bool along_eta = (edge == 0 || edge == 2);
-            T Fn[4];
-            trace_point<N1, RS, VS>((along_eta ? sG : sF) + el * FS, sOps + N1 * N1,
-                                    sOps + N1 * N1 + N1, edge, fp, Fn);
-            const T sgn = (edge == 0 || edge == 3) ? T(-1) : T(1);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) Fd[v] = ss * Fc[v] - sgn * Fn[v];
-        }
-        store4(sD + el * DS + k * 4, Fd);
+        if (face) flux_difference<P>((fl.dir ? sF : sG) + el * FP, sOps, fl, Fd);
+        store4(sD + el * DP + face_slot<P, T>(fl.dir, fl.side, fl.line), Fd);
     }
     __syncthreads();
 
     // ---- C: divergence, VCJH correction, 1/J, stage update
     double rsq = 0.0;
     if (is_sp) {
-        const long long idx = e * NSP + k;
+        const long long idx = e * NSP + ks;
         double u0[4];
         if (a.stage >= 2) gload4(a.U0 + idx * 4, u0);
-        T Di[N1], Dj[N1];
-#pragma unroll
-        for (int m = 0; m < N1; ++m) { Di[m] = sOps[i * N1 + m]; Dj[m] = sOps[j * N1 + m]; }
-        const T* gL = sOps + N1 * N1 + 2 * N1;
-        const T* gR = gL + N1;
-        const T gRi = gR[i], gLi = gL[i], gRj = gR[j], gLj = gL[j];
-        const T* f = sF + el * FS;
-        const T* h = sG + el * FS;
-        const T* d = sD + el * DS;
-        T c1[4], c3[4], c2[4], c0[4];
-        load4(d + (1 * N1 + j) * 4, c1);
-        load4(d + (3 * N1 + (N1 - 1 - j)) * 4, c3);
-        load4(d + (2 * N1 + (N1 - 1 - i)) * 4, c2);
-        load4(d + (0 * N1 + i) * 4, c0);
         const T iJ = rcp_any(Jd);
         T res[4];
+        divergence<P>(sF + el * FP, sG + el * FP, sD + el * DP, sOps, i, j, res);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            T fr[N1];
-            load_row<N1>(f + v * VS + j * RS, fr);
-            T div = T(0);
-#pragma unroll
-            for (int m = 0; m < N1; ++m) div = fma_any(Di[m], fr[m], div);
-#pragma unroll
-            for (int m = 0; m < N1; ++m) div = fma_any(Dj[m], h[v * VS + m * RS + i], div);
-            const T corr = gRi * c1[v] - gLi * c3[v] + gRj * c2[v] - gLj * c0[v];
-            res[v] = -(div + corr) * iJ;
-        }
+        for (int v = 0; v < 4; ++v) res[v] = -res[v] * iJ;
         if (a.stage == 0) {
             store_residual(a, idx, res, rsq);
         } else {
@@ -381,15 +426,13 @@ k_phys_stage(const StageArgsT<T> a) {
             double uo[4];
             rk_update(a.stage, *a.dt, us, u0, res, uo);
             gstore4(a.Uout + idx * 4, uo);
-            T* su = sU + el * FS + j * RS + i;
             T un[4];
             if constexpr (kRef) state_minus_ref(uo, ue, un);
             else {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) un[v] = T(uo[v]);
             }
-#pragma unroll
-            for (int v = 0; v < 4; ++v) su[v * VS] = un[v];
+            store4(sU + el * FP + j * RP + 4 * i, un);
             if (a.stage == 3) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) rsq += double(res[v]) * double(res[v]);
@@ -406,13 +449,18 @@ k_phys_stage(const StageArgsT<T> a) {
     // ---- D: traces of the new state
     if (is_fp) {
         T t[4];
-        trace_point<N1, RS, VS>(sU + el * FS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
+        state_trace<P>(sU + el * FP, sOps, fl, t);
         if constexpr (kRef) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) t[v] += ue[v];
         }
-        gstore4(a.Tout + (e * NFT + k) * 4, t);
-        if (boundary_condition_edge(r)) store_ghost<N1>(a, r, nr[0], nr[1], fp, t);
+        gstore4(a.Tout + (e * NFT + kf) * 4, t);
+        if (bc_face) {   // (read again: held from the loads on, they cost more)
+            const EdgeRec rb = a.edges[e * 4 + edge];
+            T n[3];
+            load_normal(normal_rec<N1>(a, e, edge, fp), n);
+            store_ghost<N1>(a, rb, n[0], n[1], fp, t);
+        }
     }
 }
 
@@ -423,11 +471,12 @@ __global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS)
 k_phys_traces(const StageArgsT<T> a) {
     using S = Shape<P, EbDiv<T>::value>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = Tiles<P, T>::FS;
-    __shared__ T sOps[S::NOPS];
-    __shared__ __align__(16) T sU[EB * FS];
+    using Op = OpTable<P + 1, T>;
+    constexpr int RP = Tiles<P, T>::RP, FP = Tiles<P, T>::FP;
+    __shared__ __align__(16) Weight<T> sOps[Op::N];
+    __shared__ __align__(16) T sU[EB * FP];
     const int tid = threadIdx.x;
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    Op::fill(sOps, a.ops);
     const int el = tid / TPE, k = tid - el * TPE;
     bool valid;
     const long long e = block_element(a, EB, el, valid);
@@ -438,21 +487,20 @@ k_phys_traces(const StageArgsT<T> a) {
         double u[4];
         T w[4];
         stage_state(a, e * NSP + k, u, w);
-        T* su = sU + el * FS + (k / N1) * RS + (k % N1);
         if constexpr (kRef) state_minus_ref(u, ue, w);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) su[v * VS] = w[v];
+        store4(sU + el * FP + (k / N1) * RP + 4 * (k % N1), w);
     }
     __syncthreads();
     if (valid && k < NFT) {
-        const int edge = k / N1, fp = k - edge * N1;
+        const FaceLane fl = lane_face<N1>(k);
+        const int edge = fl.edge, fp = fl.fp;
         T t[4];
-        trace_point<N1, RS, VS>(sU + el * FS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
+        state_trace<P>(sU + el * FP, sOps, fl, t);
         if constexpr (kRef) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) t[v] += ue[v];
         }
-        gstore4(a.Tout + (e * NFT + k) * 4, t);
+        gstore4(a.Tout + (e * NFT + edge * N1 + fp) * 4, t);
         const EdgeRec r = a.edges[e * 4 + edge];
         if (boundary_condition_edge(r)) {
             T n[3];

@@ -46,6 +46,45 @@ struct Shape {
     static constexpr int DS = 4 * NFT + 2;
 };
 
+// Solution point (i, j) of an element's thread k.  A shared-memory load of 8 or
+// 16 bytes a lane takes half the wavefronts when every aligned group of 4
+// lanes reads at most 2 distinct addresses (measured: 1 instead of 2, 2
+// instead of 4).  With points in row order a line of constant j satisfies
+// that and a line of constant i does not; with 2 x 2 patches of points on 4
+// neighbouring lanes both do.  Odd N1 has no such tiling and keeps the row
+// order.
+template <int N1>
+__device__ __forceinline__ void lane_point(int k, int& i, int& j) {
+    if constexpr (N1 % 2 == 0) {
+        const int p = k >> 2;
+        i = 2 * (p % (N1 / 2)) + (k & 1);
+        j = 2 * (p / (N1 / 2)) + ((k >> 1) & 1);
+    } else {
+        i = k % N1;
+        j = k / N1;
+    }
+}
+
+// Flux point of an element's thread k: the two ends of a line of solution
+// points sit on neighbouring lanes (they read the same tile values).  dir 0:
+// eta-lines (xi index `line`) with ends on edges 0 and 2; dir 1: xi-lines (eta
+// index `line`) with ends on edges 3 and 1; side 0 at -1, side 1 at +1.  Edges
+// run counter-clockwise, so edges 2 and 3 count their points backwards.
+struct FaceLane {
+    int dir, line, side, edge, fp;
+};
+template <int N1>
+__device__ __forceinline__ FaceLane lane_face(int k) {
+    FaceLane f;
+    f.dir = k >= 2 * N1;
+    const int t = k - f.dir * 2 * N1;
+    f.line = t >> 1;
+    f.side = t & 1;
+    f.edge = f.dir ? (f.side ? 1 : 3) : (f.side ? 2 : 0);
+    f.fp = (f.dir == f.side) ? f.line : N1 - 1 - f.line;
+    return f;
+}
+
 template <typename T>
 struct EbDiv { static constexpr int value = sizeof(T) > 8 ? 3 : 1; };
 
@@ -60,8 +99,21 @@ __device__ __forceinline__ void load4(const double* p, double* v) {
 // aligned: the library's buffers come from cudaMalloc with every row at a
 // multiple of 32 bytes, and the entry points refuse caller arrays that are
 // not 32-byte aligned.
+// load4_nc may be moved by the compiler (a pointer to what kernels write must
+// come from after_wait(), or the load could rise above griddepcontrol.wait);
+// load4_now keeps its place in the program.
 __device__ __forceinline__ void load4_nc(const double* p, double* v) {
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+__device__ __forceinline__ void load4_now(const double* p, double* v) {
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
+}
+template <typename T>
+__device__ __forceinline__ const T* after_wait(const T* p) {
+    asm volatile("" : "+l"(p));
+    return p;
 }
 __device__ __forceinline__ void gload4(const double* p, double* v) {
     asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
@@ -91,6 +143,9 @@ __device__ __forceinline__ void load4(const float* p, float* v) {
 __device__ __forceinline__ void load4_nc(const float* p, float* v) {
     const float4 a = __ldg(reinterpret_cast<const float4*>(p));
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+__device__ __forceinline__ void load4_now(const float* p, float* v) {
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p));
 }
 __device__ __forceinline__ void store4(float* p, const float* v) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
@@ -225,6 +280,164 @@ __device__ __forceinline__ void trace_point(const T* s, const T* Lm, const T* Lp
     }
 }
 
+// ---- four variables of a point, and an operator weight applied to all four.
+// Shared tiles hold points as [row][col][var], so a point is one 16-byte (FP32)
+// or two 16-byte (FP64) accesses and the operator products run over whole
+// points.  FP32 keeps the variables as two packed pairs and weights as
+// duplicated pairs: one fma.rn.f32x2 does two variables (the same rounding as
+// two scalar FMAs in half the issue slots).  Against scalar [var][row][col]
+// tiles with points in row order (stage kernels, 256 x 256, P3): FP64
+// shared-memory wavefronts halved for columns, 86 -> 79 us; FP32 warp
+// instructions 35.2 -> 30.1 M; inviscid curved P4 FP64 48 -> 40 us.
+template <typename T>
+struct V4 { T v[4]; };
+template <>
+struct V4<float> { unsigned long long a, b; };
+
+template <typename T> struct WeightOf { using type = T; };
+template <> struct WeightOf<float> { using type = unsigned long long; };
+template <typename T> using Weight = typename WeightOf<T>::type;
+
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long p, float& x, float& y) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+template <typename T> __device__ __forceinline__ Weight<T> weight(T w) { return w; }
+template <> __device__ __forceinline__ unsigned long long weight<float>(float w) { return pack2(w, w); }
+
+template <typename T>
+__device__ __forceinline__ V4<T> v4(const T* x) {
+    V4<T> r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.v[i] = x[i];
+    return r;
+}
+__device__ __forceinline__ V4<float> v4(const float* x) { return {pack2(x[0], x[1]), pack2(x[2], x[3])}; }
+template <typename T>
+__device__ __forceinline__ void v4_get(const V4<T>& a, T* x) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = a.v[i];
+}
+__device__ __forceinline__ void v4_get(const V4<float>& a, float* x) {
+    unpack2(a.a, x[0], x[1]);
+    unpack2(a.b, x[2], x[3]);
+}
+template <typename T>
+__device__ __forceinline__ V4<T> v4_zero() {
+    V4<T> r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.v[i] = T(0);
+    return r;
+}
+template <> __device__ __forceinline__ V4<float> v4_zero<float>() { return {0ull, 0ull}; }
+// acc + w x
+template <typename T>
+__device__ __forceinline__ V4<T> v4_fma(const T& w, const V4<T>& x, const V4<T>& acc) {
+    V4<T> r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.v[i] = fma_any(w, x.v[i], acc.v[i]);
+    return r;
+}
+__device__ __forceinline__ V4<float> v4_fma(unsigned long long w, const V4<float>& x, const V4<float>& acc) {
+    return {fma2(w, x.a, acc.a), fma2(w, x.b, acc.b)};
+}
+template <typename T>
+__device__ __forceinline__ V4<T> v4_mul(const T& w, const V4<T>& x) {
+    V4<T> r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r.v[i] = w * x.v[i];
+    return r;
+}
+__device__ __forceinline__ V4<float> v4_mul(unsigned long long w, const V4<float>& x) {
+    return {mul2(w, x.a), mul2(w, x.b)};
+}
+// A point of a shared tile (16-byte aligned).
+template <typename T>
+__device__ __forceinline__ V4<T> v4_load(const T* p) {
+    V4<T> r;
+    load4(p, r.v);
+    return r;
+}
+__device__ __forceinline__ V4<float> v4_load(const float* p) {
+    const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
+    return {t.x, t.y};
+}
+template <typename T>
+__device__ __forceinline__ void v4_store(T* p, const V4<T>& a) { store4(p, a.v); }
+__device__ __forceinline__ void v4_store(float* p, const V4<float>& a) {
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a.a, a.b);
+}
+
+// Weights of an operator row in shared memory.
+template <int N, typename W>
+__device__ __forceinline__ void load_weights(const W* row, W* out) {
+#pragma unroll
+    for (int m = 0; m < N; ++m) out[m] = row[m];
+}
+// 8-byte weights (double, or a duplicated float pair) of a 16-byte aligned row
+template <int N>
+__device__ __forceinline__ void load_weights(const unsigned long long* row, unsigned long long* out) {
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int m = 0; m < N; m += 2) {
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(row + m);
+            out[m] = t.x;
+            out[m + 1] = t.y;
+        }
+    } else {
+#pragma unroll
+        for (int m = 0; m < N; ++m) out[m] = row[m];
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_weights(const double* row, double* out) {
+    if constexpr (N % 2 == 0) load_row<N>(row, out);
+    else {
+#pragma unroll
+        for (int m = 0; m < N; ++m) out[m] = row[m];
+    }
+}
+
+// The 1-D operators of a kernel in shared memory, as weights: D1 rows, then
+// Lm, Lp, -Lp, gL, gR, -gL.
+template <int N1, typename T>
+struct OpTable {
+    static constexpr int LM = N1 * N1, LP = LM + N1, NLP = LP + N1, GL = NLP + N1, GR = GL + N1, NGL = GR + N1;
+    static constexpr int N = NGL + N1;
+    static __device__ __forceinline__ void fill(Weight<T>* s, const T* ops) {
+        // ops: D1, Lm, Lp, gL, gR
+        for (int t = threadIdx.x; t < N; t += blockDim.x) {
+            const bool neg = (t >= NLP && t < GL) || t >= NGL;
+            const int src = t < NLP ? t : (t < GL ? t - N1 : (t < NGL ? t - N1 : t - 3 * N1));
+            const T x = ops[src];
+            s[t] = weight<T>(neg ? -x : x);
+        }
+    }
+};
+
+// acc + sum_m w[m] (point m of a line starting at p with the given stride).
+template <int N1, typename T>
+__device__ __forceinline__ V4<T> line_dot(const Weight<T>* w, const T* p, int stride, V4<T> acc) {
+#pragma unroll
+    for (int m = 0; m < N1; ++m) acc = v4_fma(w[m], v4_load(p + m * stride), acc);
+    return acc;
+}
+
 // Programmatic dependent launch (sm_90+): a kernel launched with
 // cudaLaunchAttributeProgrammaticStreamSerialization may start while the
 // previous kernel in its stream finishes.  pdl_launch_dependents lets the
@@ -258,25 +471,6 @@ template <typename... KA, typename... AA>
 cudaError_t launch_programmatic(void (*kernel)(KA...), unsigned grid, unsigned threads, cudaStream_t s,
                                 AA&&... args) {
     return launch_programmatic_smem(kernel, grid, threads, 0, s, static_cast<AA&&>(args)...);
-}
-
-// Trace of one flux point from row `line` of a [var][row][col] tile (weights W
-// over the columns), with the row loads of load_row; the sum runs in the
-// order of trace_point, so the two agree bit for bit on the same values.
-template <int N1, int RS, int VS, typename T>
-__device__ __forceinline__ void trace_row(const T* s, const T* W, int line, T* out) {
-    T w[N1];
-#pragma unroll
-    for (int m = 0; m < N1; ++m) w[m] = W[m];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        T r[N1];
-        load_row<N1>(s + v * VS + line * RS, r);
-        T t = T(0);
-#pragma unroll
-        for (int m = 0; m < N1; ++m) t = fma_any(w[m], r[m], t);
-        out[v] = t;
-    }
 }
 
 // Block-wide deterministic sum; result valid in thread 0.

@@ -85,6 +85,7 @@ __device__ __forceinline__ void load4(const Dual* p, Dual* v) {
     }
 }
 __device__ __forceinline__ void load4_nc(const Dual* p, Dual* v) { load4(p, v); }
+__device__ __forceinline__ void load4_now(const Dual* p, Dual* v) { load4(p, v); }
 __device__ __forceinline__ void store4(Dual* p, const Dual* v) {
     double2* q = reinterpret_cast<double2*>(p);
 #pragma unroll
