@@ -4,13 +4,15 @@
 // One fused launch per RK stage.  A CTA owns EB consecutive elements; every
 // element has TPE threads.  Per stage:
 //   A  thread per solution point: load the stage state (32 contiguous bytes
-//      per point, coalesced across the warp), Euler fluxes into shared memory.
+//      per point), Euler fluxes into shared memory.
 //   B  thread per flux point: own trace + the neighbour's trace (written by
 //      the previous stage), ghost state on boundaries, Rusanov flux and the
 //      flux difference of this element's side, into shared memory.
 //   C  thread per solution point: sum-factorised divergence, FR correction,
 //      SSP-RK3 update and positivity clamp; write the new state.
 //   D  thread per flux point: traces of the new state for the next stage.
+// Bound by the shared-memory pipe (75 % of its peak with scalar tiles, 256 x 256
+// P3): the tiles and lane maps of zj_tiles.cuh took a step from 168 to 165 us.
 // The 2D reference operators are Kronecker products of 1D ones with exact
 // 0/1 factors, so the sum-factorised sums add the same nonzero terms in the
 // same order as the reference's dense loops.
@@ -23,6 +25,7 @@
 #include "zj_kernels.h"
 #include "zj_math.h"
 #include "zj_device.cuh"
+#include "zj_tiles.cuh"
 
 namespace zj {
 
@@ -196,16 +199,17 @@ __global__ void __launch_bounds__(Shape<P>::THREADS, kMinBlocks)
 k_compat_stage(const StageArgs a) {
     using S = Shape<P>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = S::FS, DS = S::DS;
-    __shared__ double sOps[S::NOPS];
-    __shared__ __align__(16) double sF[EB * FS];
-    __shared__ __align__(16) double sG[EB * FS];
-    __shared__ __align__(16) double sD[EB * DS];
-    __shared__ __align__(16) double sU[EB * FS];
+    using Op = OpTable<P + 1, double>;
+    constexpr int RP = Tiles<P, double>::RP, FP = Tiles<P, double>::FP, DP = Tiles<P, double>::DP;
+    __shared__ __align__(16) double sOps[Op::N];
+    __shared__ __align__(16) double sF[EB * FP];
+    __shared__ __align__(16) double sG[EB * FP];
+    __shared__ __align__(16) double sD[EB * DP];   // by edge point: slot (dir, side, fp)
+    __shared__ __align__(16) double sU[EB * FP];
     __shared__ double sRed[32];
 
     const int tid = threadIdx.x;
-    for (int i = tid; i < S::NOPS; i += blockDim.x) sOps[i] = a.ops[i];
+    Op::fill(sOps, a.ops);
     pdl_launch_dependents();
     pdl_wait();   // the state and traces come from the previous stage
 
@@ -215,8 +219,11 @@ k_compat_stage(const StageArgs a) {
     const bool is_sp = valid && k < NSP;
     const bool is_fp = valid && k < NFT;
     const double g = a.gamma;
-    const int edge = k / N1, fp = k - edge * N1;   // flux-point role
-    const int i = k % N1, j = k / N1;              // solution-point role (xi, eta)
+    const FaceLane fl = lane_face<N1>(k);          // flux-point role
+    const int edge = fl.edge, fp = fl.fp, kf = edge * N1 + fp;
+    int i, j;                                      // solution-point role (xi, eta)
+    lane_point<N1>(k, i, j);
+    const int ks = j * N1 + i;
 
     // ---- A: independent global loads first; Euler fluxes into shared memory
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
@@ -225,12 +232,12 @@ k_compat_stage(const StageArgs a) {
     if (is_fp) {
         r = a.edges[e * 4 + edge];
         nr = __ldg(reinterpret_cast<const double2*>(a.enrm + e * 4 + edge));
-        load4_nc(a.Tin + (e * NFT + k) * 4, qo);
+        load4_now(a.Tin + (e * NFT + kf) * 4, qo);
     }
     if (is_sp) {
-        const long long idx = e * NSP + k;
+        const long long idx = e * NSP + ks;
         gload4(a.U + idx * 4, u);
-        if ((k & 3) == 0) {
+        if ((ks & 3) == 0) {
             prefetch_l2(a.Jinv + idx * 4);
             if (a.stage >= 2) prefetch_l2(a.U0 + idx * 4);
         }
@@ -238,15 +245,15 @@ k_compat_stage(const StageArgs a) {
     // Every flux point meets the neighbour's mirrored point N1-1-fp: both
     // elements run their shared edge counter-clockwise (kernels.cu:577).
     if (is_fp && !(r.flags & (kEdgeOrphan | kEdgeBoundary)))
-        load4_nc(a.Tin + (((long long)r.nbr * 4 + r.nbr_edge) * N1 + (N1 - 1 - fp)) * 4, qn);
+        load4_now(a.Tin + (((long long)r.nbr * 4 + r.nbr_edge) * N1 + (N1 - 1 - fp)) * 4, qn);
     if (is_sp) {
         const double ir = rcp_any(u[0]);
         const double uu = u[1] * ir, vv = u[2] * ir, E = u[3] * ir;
         const double p = (g - 1.0) * u[0] * (E - 0.5 * (uu * uu + vv * vv));
-        double* f = sF + el * FS + j * RS + i;
-        double* h = sG + el * FS + j * RS + i;
-        f[0] = u[1]; f[VS] = u[1] * uu + p; f[2 * VS] = u[1] * vv; f[3 * VS] = (u[3] + p) * uu;
-        h[0] = u[2]; h[VS] = u[2] * uu; h[2 * VS] = u[2] * vv + p; h[3 * VS] = (u[3] + p) * vv;
+        const double F[4] = {u[1], u[1] * uu + p, u[1] * vv, (u[3] + p) * uu};
+        const double G[4] = {u[2], u[2] * uu, u[2] * vv + p, (u[3] + p) * vv};
+        store4(sF + el * FP + j * RP + 4 * i, F);
+        store4(sG + el * FP + j * RP + 4 * i, G);
     }
 
     // ---- B: common flux of each face point, computed once per side.  A left
@@ -258,7 +265,7 @@ k_compat_stage(const StageArgs a) {
     if (is_fp) {
         const double nx = nr.x, ny = nr.y;
         double Fc[4] = {0.0, 0.0, 0.0, 0.0};
-        int target = k;
+        int target = fp;
         if (!(r.flags & kEdgeOrphan)) {
             Prim O, X;
             make_prim(qo, g, O);
@@ -270,17 +277,17 @@ k_compat_stage(const StageArgs a) {
             rusanov_pair(O, X, right, nx, ny, Fc);
             flux_normal(O, nx, ny, Fi);   // interior flux of this point (kernels.cu:389-424)
             sig = right ? -1.0 : 1.0;
-            target = right ? edge * N1 + (N1 - 1 - fp) : k;
+            target = right ? N1 - 1 - fp : fp;
         }
         double c[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) c[v] = sig * Fc[v];
-        store4(sD + el * DS + target * 4, c);
+        store4(sD + el * DP + face_slot<P, double>(fl.dir, fl.side, target), c);
     }
     __syncthreads();   // sOps, sF, sG, common fluxes ready
     // Flux difference of this point: left Fc - Fi, right -Fc + Fi (kernels.cu:393-424).
     if (is_fp) {
-        double* d = sD + el * DS + k * 4;
+        double* d = sD + el * DP + face_slot<P, double>(fl.dir, fl.side, fp);
         double t[4];
         load4(d, t);
 #pragma unroll
@@ -292,39 +299,32 @@ k_compat_stage(const StageArgs a) {
     // ---- C: divergence, correction, stage update
     double rsq = 0.0;
     if (is_sp) {
-        const long long idx = e * NSP + k;
+        const long long idx = e * NSP + ks;
         double ji[4], u0[4];
         load4_nc(a.Jinv + idx * 4, ji);
         if (a.stage >= 2) gload4(a.U0 + idx * 4, u0);
-        double Di[N1], Dj[N1];
-#pragma unroll
-        for (int m = 0; m < N1; ++m) { Di[m] = sOps[i * N1 + m]; Dj[m] = sOps[j * N1 + m]; }
-        const double* gL = sOps + N1 * N1 + 2 * N1;
-        const double* gR = gL + N1;
-        const double gLj = gL[j], gRi = gR[i], gRj = gR[j], gLi = gL[i];
-        const double* f = sF + el * FS;
-        const double* h = sG + el * FS;
-        const double* d = sD + el * DS;
+        const double* f = sF + el * FP;
+        const double* h = sG + el * FP;
+        const double* d = sD + el * DP;
+        double w[N1], dFdxi[4], dFdeta[4], dGdxi[4], dGdeta[4];
+        load_weights<N1>(sOps + i * N1, w);
+        v4_get(line_dot<N1>(w, f + j * RP, 4, v4_zero<double>()), dFdxi);
+        v4_get(line_dot<N1>(w, h + j * RP, 4, v4_zero<double>()), dGdxi);
+        load_weights<N1>(sOps + j * N1, w);
+        v4_get(line_dot<N1>(w, f + 4 * i, RP, v4_zero<double>()), dFdeta);
+        v4_get(line_dot<N1>(w, h + 4 * i, RP, v4_zero<double>()), dGdeta);
+        const double gLj = sOps[Op::GL + j], gRi = sOps[Op::GR + i], gRj = sOps[Op::GR + j], gLi = sOps[Op::GL + i];
+        // the reference pairs every edge's point number with the solution
+        // point's own index, edges 2 and 3 (which run backwards) included
         double c0[4], c1[4], c2[4], c3[4];
-        load4(d + (0 * N1 + i) * 4, c0);
-        load4(d + (1 * N1 + j) * 4, c1);
-        load4(d + (2 * N1 + i) * 4, c2);
-        load4(d + (3 * N1 + j) * 4, c3);
+        load4(d + face_slot<P, double>(0, 0, i), c0);
+        load4(d + face_slot<P, double>(1, 1, j), c1);
+        load4(d + face_slot<P, double>(0, 1, i), c2);
+        load4(d + face_slot<P, double>(1, 0, j), c3);
         double res[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            double fr[N1], gr[N1];
-            load_row<N1>(f + v * VS + j * RS, fr);
-            load_row<N1>(h + v * VS + j * RS, gr);
-            double dFdxi = 0.0, dFdeta = 0.0, dGdxi = 0.0, dGdeta = 0.0;
-#pragma unroll
-            for (int m = 0; m < N1; ++m) {
-                dFdxi = fma(Di[m], fr[m], dFdxi);
-                dFdeta = fma(Dj[m], f[v * VS + m * RS + i], dFdeta);
-                dGdxi = fma(Di[m], gr[m], dGdxi);
-                dGdeta = fma(Dj[m], h[v * VS + m * RS + i], dGdeta);
-            }
-            const double div = (dFdxi * ji[0] + dFdeta * ji[2]) + (dGdxi * ji[1] + dGdeta * ji[3]);
+            const double div = (dFdxi[v] * ji[0] + dFdeta[v] * ji[2]) + (dGdxi[v] * ji[1] + dGdeta[v] * ji[3]);
             double rr = -div;
             double corr = 0.0;
             corr += c0[v] * gLj;
@@ -349,9 +349,7 @@ k_compat_stage(const StageArgs a) {
             }
             positivity(uo);
             gstore4(a.Uout + idx * 4, uo);
-            double* su = sU + el * FS + j * RS + i;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) su[v * VS] = uo[v];
+            store4(sU + el * FP + j * RP + 4 * i, uo);
             if (a.stage == 3) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) rsq += res[v] * res[v];
@@ -368,8 +366,8 @@ k_compat_stage(const StageArgs a) {
     // ---- D: traces of the new state
     if (is_fp) {
         double t[4];
-        trace_point<N1, RS, VS>(sU + el * FS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
-        gstore4(a.Tout + (e * NFT + k) * 4, t);
+        state_trace<P>(sU + el * FP, sOps, fl, t);
+        gstore4(a.Tout + (e * NFT + kf) * 4, t);
     }
 }
 
@@ -379,36 +377,54 @@ k_traces(const double* __restrict__ U, double* __restrict__ T, const double* __r
          long long n_elem) {
     using S = Shape<P>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int RS = S::RS, VS = S::VS, FS = S::FS;
-    __shared__ double sOps[S::NOPS];
-    __shared__ double sU[EB * FS];
+    using Op = OpTable<P + 1, double>;
+    constexpr int RP = Tiles<P, double>::RP, FP = Tiles<P, double>::FP;
+    __shared__ __align__(16) double sOps[Op::N];
+    __shared__ __align__(16) double sU[EB * FP];
     const int tid = threadIdx.x;
-    for (int i = tid; i < S::NOPS; i += blockDim.x) sOps[i] = ops[i];
+    Op::fill(sOps, ops);
     const int el = tid / TPE, k = tid - el * TPE;
     const long long e = (long long)blockIdx.x * EB + el;
     const bool valid = (el < EB) && (e < n_elem);
     if (valid && k < NSP) {
         double u[4];
         load4_nc(U + (e * NSP + k) * 4, u);
-        double* su = sU + el * FS + (k / N1) * RS + (k % N1);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) su[v * VS] = u[v];
+        store4(sU + el * FP + (k / N1) * RP + 4 * (k % N1), u);
     }
     __syncthreads();
     if (valid && k < NFT) {
-        const int edge = k / N1, fp = k - edge * N1;
+        const FaceLane fl = lane_face<N1>(k);
         double t[4];
-        trace_point<N1, RS, VS>(sU + el * FS, sOps + N1 * N1, sOps + N1 * N1 + N1, edge, fp, t);
-        gstore4(T + (e * NFT + k) * 4, t);
+        state_trace<P>(sU + el * FP, sOps, fl, t);
+        gstore4(T + (e * NFT + fl.edge * N1 + fl.fp) * 4, t);
     }
 }
 
-__global__ void k_reduce_sum(const double* __restrict__ x, int n, double* out) {
+// out = sum of x, or out += w * sum of x (accumulate), in a fixed order.  One
+// block: four independent loads a round and shuffles at both levels, since
+// the few thousand partials cost latency only.
+__global__ void k_reduce_sum(const double* __restrict__ x, int n, double* out, double w, bool accumulate) {
     __shared__ double red[32];
-    double s = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) s += x[i];
-    const double t = block_sum(s, red);
-    if (threadIdx.x == 0) out[0] = t;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    const int b = blockDim.x;
+    int i = threadIdx.x;
+    for (; i + 3 * b < n; i += 4 * b) {
+        s0 += x[i];
+        s1 += x[i + b];
+        s2 += x[i + 2 * b];
+        s3 += x[i + 3 * b];
+    }
+    for (; i < n; i += b) s0 += x[i];
+    double s = (s0 + s1) + (s2 + s3);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    s = (threadIdx.x < (unsigned)(b >> 5)) ? red[threadIdx.x] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (threadIdx.x == 0) out[0] = accumulate ? out[0] + w * s : s;
 }
 
 __global__ void k_dt_partial(const double* __restrict__ U, const double* __restrict__ h,
@@ -527,7 +543,12 @@ cudaError_t launch_traces(int P, const double* U, double* T, const double* ops, 
 }
 
 cudaError_t launch_reduce_sum(const double* partials, int n, double* out, cudaStream_t s) {
-    k_reduce_sum<<<1, 1024, 0, s>>>(partials, n, out);
+    k_reduce_sum<<<1, 1024, 0, s>>>(partials, n, out, 1.0, false);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_reduce_add(const double* partials, int n, double w, double* out, cudaStream_t s) {
+    k_reduce_sum<<<1, 1024, 0, s>>>(partials, n, out, w, true);
     return cudaGetLastError();
 }
 
