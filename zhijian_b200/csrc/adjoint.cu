@@ -30,8 +30,12 @@
 #include "ns_kernels.cuh"
 #include "zj_adjoint.cuh"
 
+// Navier-Stokes adjoint kernel: 250 registers and 4 CTAs of 64 threads per SM,
+// no spills.  168 registers and 6 CTAs spill 500 bytes; on 91 x 57 quads (P2, one
+// wave) a Gauss-Newton product then takes 97 us instead of 87, on 128 x 128
+// (P3) eight adjoint steps 3.46 ms instead of 3.48.
 #ifndef ZJ_ADJ_MIN_BLOCKS
-#define ZJ_ADJ_MIN_BLOCKS 3       // Navier-Stokes adjoint kernel (168 registers)
+#define ZJ_ADJ_MIN_BLOCKS 2
 #endif
 
 namespace zj {
@@ -275,7 +279,7 @@ k_adj_ns(const AdjArgs a) {
     const bool is_sp = valid && k < NSP, is_fp = valid && k < NFT;
     const int edge = k / N1, fp = k - edge * N1;
     const int i = k % N1, j = k / N1;
-    const double g = a.gamma, Re = a.Re, Pr = a.Pr;
+    const double g = a.gamma, iRe = a.iRe, kfac = a.kfac;
 
     // ---- 1: loads
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
@@ -338,7 +342,7 @@ k_adj_ns(const AdjArgs a) {
             mGb[v] = -Gb[v];
         }
         adj::euler_flux_vjp(u, g, Fb, Gb, ub);
-        re_acc -= adj::viscous_vjp(u, Qx, Qy, g, Re, Pr, mFb, mGb, ub, Qxb, Qyb) / Re;
+        re_acc -= adj::viscous_vjp(u, Qx, Qy, g, iRe, kfac, mFb, mGb, ub, Qxb, Qyb) * iRe;
     }
     double tb[4] = {0.0, 0.0, 0.0, 0.0};
     if (is_fp) {
@@ -369,8 +373,8 @@ k_adj_ns(const AdjArgs a) {
                 Fvb[v] = -Fnb[v] * nx;
                 Gvb[v] = -Fnb[v] * ny;
             }
-            const double dv = adj::viscous_vjp(Ua, dxa, dya, g, Re, Pr, Fvb, Gvb, Uab, dxb, dyb);
-            if (!right) re_acc -= dv / Re;   // once per face: on its left element
+            const double dv = adj::viscous_vjp(Ua, dxa, dya, g, iRe, kfac, Fvb, Gvb, Uab, dxb, dyb);
+            if (!right) re_acc -= dv * iRe;   // once per face: on its left element
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 ULb[v] += 0.5 * Uab[v];

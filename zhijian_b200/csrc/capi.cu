@@ -110,6 +110,8 @@ struct zj_solver {
     double* aDot = nullptr;     // dot-product partials
     double* aScal = nullptr;    // [0] dJ/dRe accumulator, [1] dot result
     double* aRePart = nullptr;  // per-CTA L . dR/dRe of the NS VJP
+    double* aWork = nullptr;    // checkpoints and segment of zj_adjoint_run, kept up to kAdjKeepBytes
+    size_t aWork_n = 0;
     int grid = 0;
     int cur = 0, tpar = 0;
     bool traces_valid = false;
@@ -188,9 +190,11 @@ void free_all(zj_solver* s) {
     s->dElistQ = s->dElistT = nullptr; s->dTriOps = nullptr; s->fTriOps = nullptr; s->dEtype = nullptr;
     void* xs[] = {s->xJinv, s->xJ, s->xOps, s->xBC, s->xNrm, s->xT, s->xTQ, s->xPart, s->aDb, s->aTb,
                   s->aDUb, s->aW, s->aS1, s->aS2, s->aB0, s->aB1, s->aB2, s->aR, s->aJV, s->aZero,
-                  s->aDot, s->aScal, s->aRePart};
+                  s->aDot, s->aScal, s->aRePart, s->aWork};
     for (void* p : xs) if (p) cudaFree(p);
     s->diff_ready = false;
+    s->aWork = nullptr;
+    s->aWork_n = 0;
     if (s->dFlag) cudaFree(s->dFlag);
     if (s->dEdges) cudaFree(s->dEdges);
     if (s->dNrm) cudaFree(s->dNrm);
@@ -1014,6 +1018,9 @@ zj_status zj_rhs_noalloc(zj_solver* s, const double* U_dev, double* R_dev) {
 // adjoint of a run.
 namespace {
 
+// What a handle keeps allocated between zj_adjoint_run calls, at most.
+constexpr size_t kAdjKeepBytes = size_t(1) << 30;
+
 zj_status diff_supported(zj_solver* s) {
     if (s->prm.compat) return fail(s, ZJ_ERR_UNSUPPORTED, "differentiation needs physics mode (compat off)");
     if (s->mixed) return fail(s, ZJ_ERR_UNSUPPORTED, "differentiation runs on the FP64 path (precision fp64)");
@@ -1111,16 +1118,15 @@ zj_status vjp_core(zj_solver* s, const double* U, const double* L, double* W, do
     g.U = U; g.L = L; g.W = W; g.T = T; g.TQ = TQ;
     g.Db = s->aDb; g.Tb = s->aTb; g.DUb = s->aDUb;
     g.Jinv = s->dJinv; g.J = s->dJ; g.edges = s->dEdges; g.enrm = s->dNrm; g.bc = s->dBC; g.ops = s->dOps;
-    g.n_elem = s->E; g.gamma = s->prm.gamma; g.Re = s->prm.Re; g.Pr = s->prm.Pr;
+    g.n_elem = s->E; g.gamma = s->prm.gamma;
+    g.iRe = 1.0 / s->prm.Re; g.kfac = g.gamma / ((g.gamma - 1.0) * s->prm.Pr);
     const bool re = is_ns(s) && re_weight != 0.0;
     g.re_part = re ? s->aRePart : nullptr;
     g.out = o.out; g.X0 = o.X0; g.X1 = o.X1; g.X2 = o.X2;
     g.c0 = o.c0; g.c1 = o.c1; g.c2 = o.c2; g.cw = o.cw;
     ZJ_CK(s, launch_rhs_vjp(s->P, s->prm.riemann, is_ns(s), g, s->stream), "vjp launch");
     if (re) {
-        ZJ_CK(s, launch_reduce_sum(s->aRePart, adj_ns_grid(s->P, s->E), s->aScal + 1, s->stream), "re reduce");
-        ZJ_CK(s, launch_lincomb(s->aScal, 1.0, s->aScal, re_weight, s->aScal + 1, 0.0, nullptr, 1, s->stream),
-              "re accumulate");
+        ZJ_CK(s, launch_reduce_add(s->aRePart, adj_ns_grid(s->P, s->E), re_weight, s->aScal, s->stream), "re reduce");
     }
     return ZJ_OK;
 }
@@ -1270,27 +1276,44 @@ zj_status zj_adjoint_run(zj_solver* s, double dt, int nsteps, int k_ckpt, double
     const int n_ck = (nsteps + k_ckpt - 1) / k_ckpt;
     const int seg_n = std::min(k_ckpt, nsteps);
     const size_t sb = s->state_n * sizeof(double);
-    double* ck = nullptr;    // checkpoints [n_ck][state]
-    double* seg = nullptr;   // step-start states of one segment [seg_n][state]
-    double* X = nullptr;     // forward work state
     // per step of a segment: 3 states, and 3 trace sets (traces + gradient
     // traces) of the stage inputs
     const size_t tset = s->trace_n * (is_ns(s) ? 3 : 1);
-    double* trs = nullptr;
-    cudaError_t e = dalloc(&ck, (size_t)n_ck * s->state_n);
-    if (e == cudaSuccess) e = dalloc(&seg, (size_t)3 * seg_n * s->state_n);
-    if (e == cudaSuccess) e = dalloc(&trs, (size_t)3 * seg_n * tset);
-    if (e == cudaSuccess) e = dalloc(&X, s->state_n);
+    // one block: checkpoints [n_ck][state], one segment's states [3 seg_n]
+    // [state] (step start, U(1), U(2)), its trace sets [3 seg_n][tset] and the
+    // forward work state.  state_n and trace_n are multiples of 4, so every
+    // part starts on a 32-byte boundary.  The handle keeps a block of up to
+    // kAdjKeepBytes for its next run: allocating and freeing 0.4 GB a call
+    // cost 1.5 to 5 ms beside 4 ms of kernels (128 x 128, P3, 8 steps);
+    // larger ones, whose run is long, are freed at the end as they would
+    // otherwise hold memory the caller may need.
+    const size_t n_work = ((size_t)n_ck + 3 * (size_t)seg_n + 1) * s->state_n + (size_t)3 * seg_n * tset;
+    cudaError_t e = cudaSuccess;
+    if (s->aWork_n < n_work) {
+        if (s->aWork) cudaFree(s->aWork);
+        s->aWork = nullptr;
+        s->aWork_n = 0;
+        e = dalloc(&s->aWork, n_work);
+        if (e == cudaSuccess) s->aWork_n = n_work;
+    }
+    double* ck = s->aWork;
+    double* seg = ck + (size_t)n_ck * s->state_n;
+    double* trs = seg + (size_t)3 * seg_n * s->state_n;
+    double* X = trs + (size_t)3 * seg_n * tset;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     for (int i = 0; i < 4 && e == cudaSuccess; ++i) e = cudaEventCreate(&ev[i]);
-    auto cleanup = [&]() {
+    auto cleanup = [&](bool failed) {
+        // after a failure launches may still be queued: nothing of theirs may
+        // outlive the call in a block the next run writes from another stream
+        if (failed) (void)cudaStreamSynchronize(s->stream);
         for (auto x : ev) if (x) cudaEventDestroy(x);
-        if (ck) cudaFree(ck);
-        if (seg) cudaFree(seg);
-        if (trs) cudaFree(trs);
-        if (X) cudaFree(X);
+        if (s->aWork && (failed || s->aWork_n * sizeof(double) > kAdjKeepBytes)) {
+            cudaFree(s->aWork);
+            s->aWork = nullptr;
+            s->aWork_n = 0;
+        }
     };
-    if (e != cudaSuccess) { cleanup(); return cuda_fail(s, e, "adjoint checkpoint buffers"); }
+    if (e != cudaSuccess) { cleanup(true); return cuda_fail(s, e, "adjoint checkpoint buffers"); }
     const long long n = (long long)s->state_n;
     auto run = [&]() -> zj_status {
         zj_status r = ZJ_OK;
@@ -1372,7 +1395,7 @@ zj_status zj_adjoint_run(zj_solver* s, double dt, int nsteps, int k_ckpt, double
                 *bytes = (int64_t)((size_t)(n_ck + 3 * seg_n + 1 + 9) * sb + (size_t)3 * seg_n * tset * 8);
         }
     }
-    cleanup();
+    cleanup(st != ZJ_OK);
     return st;
 }
 

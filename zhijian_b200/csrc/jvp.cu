@@ -47,18 +47,6 @@ __global__ void k_to_dual(const double* __restrict__ x, Dual* __restrict__ y, lo
         y[i] = Dual(x[i], 0.0);
 }
 
-// out = a x + b y + c z (y, z may be NULL when their weight is 0)
-__global__ void k_lincomb(double* __restrict__ out, double a, const double* x, double b,
-                          const double* y, double c, const double* z, long long n) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (long long)gridDim.x * blockDim.x) {
-        double r = a * x[i];
-        if (y) r += b * y[i];
-        if (z) r += c * z[i];
-        out[i] = r;
-    }
-}
-
 // Per-CTA partial dot products with a fixed grid (deterministic order).
 __global__ void k_dot_partial(const double* __restrict__ x, const double* __restrict__ y,
                               long long n, double* partials) {
@@ -78,13 +66,6 @@ constexpr int kFillGrid = 148 * 8;
 cudaError_t launch_to_dual(const double* x, Dual* y, long long n, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     k_to_dual<<<kFillGrid, 256, 0, s>>>(x, y, n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_lincomb(double* out, double a, const double* x, double b, const double* y,
-                           double c, const double* z, long long n, cudaStream_t s) {
-    if (n <= 0) return cudaSuccess;
-    k_lincomb<<<kFillGrid, 256, 0, s>>>(out, a, x, b, y, c, z, n);
     return cudaGetLastError();
 }
 

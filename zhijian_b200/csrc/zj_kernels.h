@@ -109,8 +109,6 @@ cudaError_t launch_ns_stage_tc(int P, int riemann, const StageArgs32& a, const v
 int quad_grid(int P, long long n);
 // Elementwise helpers of the differentiation entry points (jvp.cu).
 cudaError_t launch_to_dual(const double* x, Dual* y, long long n, cudaStream_t s);
-cudaError_t launch_lincomb(double* out, double a, const double* x, double b, const double* y,
-                           double c, const double* z, long long n, cudaStream_t s);
 int dot_grid();
 // out[0] = x . y, deterministic (fixed grid; partials has dot_grid() entries).
 cudaError_t launch_dot(const double* x, const double* y, long long n, double* partials,
@@ -138,7 +136,8 @@ struct AdjArgs {
     const double* bc;
     const double* ops;
     long long n_elem;
-    double gamma, Re, Pr;
+    double gamma;
+    double iRe, kfac;       // 1/Re and gamma/((gamma-1) Pr) of the viscosity law
     double* re_part;        // optional, Navier-Stokes: per-CTA L . dR/dRe, adj_ns_grid entries
     // optional fused output: out = c0 X0 + c1 X1 + c2 X2 + cw (dR/dU)^T L
     // (an SSP-RK3 stage's adjoint update; X* may be NULL when c* is 0, out may
@@ -154,6 +153,8 @@ int adj_ns_grid(int P, long long n_elem);
 
 // Deterministic reduction of per-CTA partial sums into out[0].
 cudaError_t launch_reduce_sum(const double* partials, int n, double* out, cudaStream_t s);
+// out[0] += w * that sum.
+cudaError_t launch_reduce_add(const double* partials, int n, double w, double* out, cudaStream_t s);
 // out[0] = min over states of CFL*h/(ws*(2P+1)); h per element.
 // Triangles (etype[e] == ZJ_ELEM_TRI) count their first nt slots only.
 cudaError_t launch_compute_dt(const double* U, const double* h, long long n_elem, int n_sp,
