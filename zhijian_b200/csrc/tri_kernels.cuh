@@ -21,11 +21,17 @@
 
 #include "ns_kernels.cuh"
 
+// 128-thread CTAs: more of them sit in different phases, and the last wave is
+// finer (shear layer per step, 256 -> 128 threads: 384 x 384 P3 FP32 754 -> 734 us
+// with 64 instead of 80 registers, 173 x 141 P2 FP64 221 -> 210 us).
+#ifndef ZJ_TRI_THREADS
+#define ZJ_TRI_THREADS 128
+#endif
 #ifndef ZJ_TRI_MIN_BLOCKS
-#define ZJ_TRI_MIN_BLOCKS 2       // FP64 stage kernel (128 registers; viscous: spills of 16-36 B)
+#define ZJ_TRI_MIN_BLOCKS 4       // FP64 stage kernel (128 registers)
 #endif
 #ifndef ZJ_TRI32_MIN_BLOCKS
-#define ZJ_TRI32_MIN_BLOCKS 3     // precision-form stage kernel (80 registers)
+#define ZJ_TRI32_MIN_BLOCKS 8     // precision-form stage kernel (64 registers)
 #endif
 
 namespace zj {
@@ -34,6 +40,13 @@ namespace {
 template <typename T> struct TriMinBlocks { static constexpr int stage = ZJ_TRI_MIN_BLOCKS; };
 template <> struct TriMinBlocks<float> { static constexpr int stage = ZJ_TRI32_MIN_BLOCKS; };
 
+// Shared layout.  Field tiles are [element][point][var], so a point is one or
+// two 16-byte loads that the element's threads share; the operators' rows sit
+// by thread: (Dr, Ds) pairs of a point's row, rows of L and of Phi, padded so
+// that the rows of neighbouring threads fall on distinct banks.
+// With scalar tiles and unpaired rows the products took 5 to 6 shared loads for
+// 8 FMAs; the stage launch of 42 000 P3 triangles issued 51.7 M warp
+// instructions in FP32 and now 36.7 M.
 template <int P, typename T>
 struct TriShape {
     static constexpr int N1 = P + 1;
@@ -41,12 +54,28 @@ struct TriShape {
     static constexpr int NSP = N1 * N1;                // state slots per element
     static constexpr int NFT = 3 * N1;                 // flux points
     static constexpr int TPE = NT > NFT ? NT : NFT;
-    static constexpr int EB = (256 / TPE / EbDiv<T>::value) > 0 ? (256 / TPE / EbDiv<T>::value) : 1;
+    static constexpr int EB = (ZJ_TRI_THREADS / TPE / EbDiv<T>::value) > 0 ? (ZJ_TRI_THREADS / TPE / EbDiv<T>::value) : 1;
     static constexpr int THREADS = EB * TPE;
-    static constexpr int NOPS = 2 * NT * NT + 2 * NT * NFT;   // Dr, Ds, L, Phi
-    static constexpr int FS = NT + ((NT & 1) ? 1 : 0);        // one variable's field
-    static constexpr int ES = 4 * FS + 2;                     // element stride of a 4-variable field
-    static constexpr int DS = 4 * NFT + (sizeof(T) == 8 ? 2 : 4);
+    static constexpr int ES = 4 * NT + (sizeof(T) == 8 ? 2 : 4);    // element stride of a field tile
+    static constexpr int DS = 4 * NFT + (sizeof(T) == 8 ? 2 : 4);   // and of the flux-point tile
+    static constexpr int RD = 2 * NT + ((2 * NT) % 4 == 0 ? 2 : 4); // row strides: (Dr, Ds)
+    static constexpr int RL = NT | 1, RF = NFT | 1;                 // L, Phi
+    static constexpr int LO = NT * RD, PHI = LO + NFT * RL;
+    static constexpr int NOPS = PHI + NT * RF;
+    // packed operators (Dr, Ds, L, Phi, each row-major) into the rows above
+    static __device__ __forceinline__ void fill(T* s, const T* ops) {
+        for (int t = threadIdx.x; t < NT * NT; t += THREADS) {
+            const int n = t / NT, k = t - n * NT;
+            s[n * RD + 2 * k] = ops[t];
+            s[n * RD + 2 * k + 1] = ops[NT * NT + t];
+        }
+        for (int t = threadIdx.x; t < NFT * NT; t += THREADS) {
+            const int q = t / NT, k = t - q * NT;
+            s[LO + q * RL + k] = ops[2 * NT * NT + t];
+            const int n = t / NFT, p = t - n * NFT;
+            s[PHI + n * RF + p] = ops[2 * NT * NT + NFT * NT + t];
+        }
+    }
 };
 
 // reference-edge unit outward normals and lengths
@@ -54,57 +83,52 @@ __device__ __forceinline__ double tri_nref_x(int f) { return f == 1 ? 0.70710678
 __device__ __forceinline__ double tri_nref_y(int f) { return f == 0 ? -1.0 : (f == 1 ? 0.70710678118654752440 : 0.0); }
 __device__ __forceinline__ double tri_ref_len(int f) { return f == 1 ? 2.82842712474619009760 : 2.0; }
 
-// Interpolation of a [var][NT] field (stride FS) to flux point q.
-template <int NT, int FS, typename T>
-__device__ __forceinline__ void tri_interp(const T* fld, const T* Lrow, T* out) {
+// sum_k w[k] (point k of a field tile).
+template <int NT, typename T>
+__device__ __forceinline__ V4<T> tri_dot(const T* fld, const T* w) {
+    V4<T> acc = v4_zero<T>();
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        T t = T(0);
-#pragma unroll
-        for (int k = 0; k < NT; ++k) t = fma_any(Lrow[k], fld[v * FS + k], t);
-        out[v] = t;
-    }
+    for (int k = 0; k < NT; ++k) acc = v4_fma(weight<T>(w[k]), v4_load(fld + 4 * k), acc);
+    return acc;
 }
 
-// Corrected reference gradient at solution point n from the state field su
-// ([var][NT]) and the face jumps du ([q][var]).
-template <int NT, int NFT, int FS, typename T>
-__device__ __forceinline__ void tri_gradient(const T* su, const T* du, const T* Dr, const T* Ds,
-                                             const T* Phi, int n, const T* ji, T* Qx, T* Qy) {
-    T dr[4] = {T(0), T(0), T(0), T(0)}, ds[4] = {T(0), T(0), T(0), T(0)};
+// (Dr_k, Ds_k) of a row.
+__device__ __forceinline__ void load_pair(const float* p, float& a, float& b) {
+    const float2 t = *reinterpret_cast<const float2*>(p);
+    a = t.x; b = t.y;
+}
+__device__ __forceinline__ void load_pair(const double* p, double& a, double& b) {
+    const double2 t = *reinterpret_cast<const double2*>(p);
+    a = t.x; b = t.y;
+}
+
+// Corrected reference gradient at solution point n from the state tile su and
+// the face jumps du, chain rule with ji.  The corrections of an edge share its
+// reference normal, so they are summed per edge first.
+template <int P, typename T>
+__device__ __forceinline__ void tri_gradient(const T* su, const T* du, const T* ops, int n, const T* ji, T* Qx,
+                                             T* Qy) {
+    using S = TriShape<P, T>;
+    constexpr int NT = S::NT, N1 = S::N1;
+    V4<T> dr = v4_zero<T>(), ds = v4_zero<T>();
 #pragma unroll
     for (int k = 0; k < NT; ++k) {
-        const T a = Dr[n * NT + k], b = Ds[n * NT + k];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            dr[v] = fma_any(a, su[v * FS + k], dr[v]);
-            ds[v] = fma_any(b, su[v * FS + k], ds[v]);
-        }
+        T a, b;
+        load_pair(ops + n * S::RD + 2 * k, a, b);
+        const V4<T> u = v4_load(su + 4 * k);
+        dr = v4_fma(weight<T>(a), u, dr);
+        ds = v4_fma(weight<T>(b), u, ds);
     }
+    const T* ph = ops + S::PHI + n * S::RF;
 #pragma unroll
-    for (int q = 0; q < NFT; ++q) {
-        const int f = q / (NFT / 3);
-        const T ph = Phi[n * NFT + q];
-        const T px = ph * T(tri_nref_x(f)), py = ph * T(tri_nref_y(f));
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            dr[v] = fma_any(px, du[q * 4 + v], dr[v]);
-            ds[v] = fma_any(py, du[q * 4 + v], ds[v]);
-        }
+    for (int f = 0; f < 3; ++f) {
+        const V4<T> c = tri_dot<N1>(du + f * N1 * 4, ph + f * N1);
+        if (f > 0) dr = v4_fma(weight<T>(T(tri_nref_x(f))), c, dr);
+        if (f < 2) ds = v4_fma(weight<T>(T(tri_nref_y(f))), c, ds);
     }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-        Qx[v] = ji[0] * dr[v] + ji[2] * ds[v];
-        Qy[v] = ji[1] * dr[v] + ji[3] * ds[v];
-    }
+    v4_get(v4_fma(weight<T>(ji[2]), ds, v4_mul(weight<T>(ji[0]), dr)), Qx);
+    v4_get(v4_fma(weight<T>(ji[3]), ds, v4_mul(weight<T>(ji[1]), dr)), Qy);
 }
-
-template <int P, typename T>
-struct TriLayout {
-    using S = TriShape<P, T>;
-    // offsets in the operator tile
-    static constexpr int DR = 0, DSo = S::NT * S::NT, L = 2 * S::NT * S::NT, PHI = L + S::NFT * S::NT;
-};
 
 // Element of thread group el in this CTA, or -1.
 __device__ __forceinline__ long long tri_element(const int32_t* elist, long long n_list, int EB, int el) {
@@ -117,13 +141,11 @@ template <int P, typename T>
 __global__ void __launch_bounds__(TriShape<P, T>::THREADS)
 k_tri_traces(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n_list) {
     using S = TriShape<P, T>;
-    using Lo = TriLayout<P, T>;
-    constexpr int N1 = S::N1, NT = S::NT, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int FS = S::FS, ES = S::ES;
-    __shared__ T sOps[S::NOPS];
+    constexpr int N1 = S::N1, NT = S::NT, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB, ES = S::ES;
+    __shared__ __align__(16) T sOps[S::NOPS];
     __shared__ __align__(16) T sU[EB * ES];
     const int tid = threadIdx.x;
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    S::fill(sOps, a.ops);
     const int el = tid / TPE, k = tid - el * TPE;
     const long long e = (el < EB) ? tri_element(elist, n_list, EB, el) : -1;
     const bool valid = e >= 0;
@@ -135,14 +157,13 @@ k_tri_traces(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long
         T w[4];
         stage_state(a, e * NSP + k, u, w);
         if constexpr (kRef) state_minus_ref(u, ue, w);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) sU[el * ES + v * FS + k] = w[v];
+        store4(sU + el * ES + 4 * k, w);
     }
     __syncthreads();
     if (valid && k < NFT) {
         const int edge = k / N1, fp = k - edge * N1;
         T t[4];
-        tri_interp<NT, FS>(sU + el * ES, sOps + Lo::L + k * NT, t);
+        v4_get(tri_dot<NT>(sU + el * ES, sOps + S::LO + k * S::RL), t);
         if constexpr (kRef) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) t[v] += ue[v];
@@ -162,15 +183,14 @@ template <int P, typename T>
 __global__ void __launch_bounds__(TriShape<P, T>::THREADS)
 k_tri_grad(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n_list) {
     using S = TriShape<P, T>;
-    using Lo = TriLayout<P, T>;
     constexpr int N1 = S::N1, NT = S::NT, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int FS = S::FS, ES = S::ES, DS = S::DS;
-    __shared__ T sOps[S::NOPS];
-    __shared__ __align__(16) T sU[EB * ES];
+    constexpr int ES = S::ES, DS = S::DS;
+    __shared__ __align__(16) T sOps[S::NOPS];
+    __shared__ __align__(16) T sU[EB * ES];    // the state, then dU/dy
     __shared__ __align__(16) T sDU[EB * DS];
-    __shared__ __align__(16) T sQ[EB * 2 * ES];
+    __shared__ __align__(16) T sQ[EB * ES];    // dU/dx
     const int tid = threadIdx.x;
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    S::fill(sOps, a.ops);
     pdl_launch_dependents();
     pdl_wait();   // the state and traces come from the previous launches
     const int el = tid / TPE, k = tid - el * TPE;
@@ -179,6 +199,7 @@ k_tri_grad(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n
     const bool is_sp = valid && k < NT, is_fp = valid && k < NFT;
     const int edge = k / N1, fp = k - edge * N1;
     constexpr bool kRef = UsesRef<T>::value;
+    const T* Tin = after_wait(a.Tin);
     T ji[4];
     if (is_sp) {
         const long long idx = e * NSP + k;
@@ -191,18 +212,17 @@ k_tri_grad(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n
             state_minus_ref(ud, ue, u);
         }
         load4_nc(a.Jinv + idx * 4, ji);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) sU[el * ES + v * FS + k] = u[v];
+        store4(sU + el * ES + 4 * k, u);
     }
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
     T Ua[4];   // average state of the flux point
     if (is_fp) {
         r = a.edges[e * 4 + edge];
         T qn[4];
-        load4_nc(a.Tin + (e * 4 * N1 + k) * 4, Ua);
+        load4_nc(Tin + (e * 4 * N1 + k) * 4, Ua);
         T d[4] = {T(0), T(0), T(0), T(0)};
         if (!(r.flags & kEdgeOrphan)) {
-            load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
+            load4_nc(Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 d[v] = T(0.5) * (qn[v] - Ua[v]);
@@ -212,21 +232,18 @@ k_tri_grad(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n
         store4(sDU + el * DS + k * 4, d);
     }
     __syncthreads();
+    T Qx[4], Qy[4];
     if (is_sp) {
-        T Qx[4], Qy[4];
-        tri_gradient<NT, NFT, FS>(sU + el * ES, sDU + el * DS, sOps + Lo::DR, sOps + Lo::DSo, sOps + Lo::PHI, k,
-                                  ji, Qx, Qy);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            sQ[el * 2 * ES + v * FS + k] = Qx[v];
-            sQ[el * 2 * ES + ES + v * FS + k] = Qy[v];
-        }
+        tri_gradient<P>(sU + el * ES, sDU + el * DS, sOps, k, ji, Qx, Qy);
+        store4(sQ + el * ES + 4 * k, Qx);
     }
+    __syncthreads();   // the state tile is dead
+    if (is_sp) store4(sU + el * ES + 4 * k, Qy);
     __syncthreads();
     if (is_fp) {
         T t[8];
-        tri_interp<NT, FS>(sQ + el * 2 * ES, sOps + Lo::L + k * NT, t);
-        tri_interp<NT, FS>(sQ + el * 2 * ES + ES, sOps + Lo::L + k * NT, t + 4);
+        v4_get(tri_dot<NT>(sQ + el * ES, sOps + S::LO + k * S::RL), t);
+        v4_get(tri_dot<NT>(sU + el * ES, sOps + S::LO + k * S::RL), t + 4);
         T n[3], f[4];
         load_normal(a.enrm + e * 4 + edge, n);
         viscous_share(a, r, n[0], n[1], Ua, t, f);
@@ -239,17 +256,16 @@ template <int P, int RIEM, bool VISC, typename T>
 __global__ void __launch_bounds__(TriShape<P, T>::THREADS, TriMinBlocks<T>::stage)
 k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long n_list) {
     using S = TriShape<P, T>;
-    using Lo = TriLayout<P, T>;
     constexpr int N1 = S::N1, NT = S::NT, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
-    constexpr int FS = S::FS, ES = S::ES, DS = S::DS;
-    __shared__ T sOps[S::NOPS];
+    constexpr int ES = S::ES, DS = S::DS;
+    __shared__ __align__(16) T sOps[S::NOPS];
     __shared__ __align__(16) T sF[EB * ES];
     __shared__ __align__(16) T sG[EB * ES];
     __shared__ __align__(16) T sD[EB * DS];    // face jumps of U (NS), then flux differences
     __shared__ __align__(16) T sU[EB * ES];    // stage state (NS), then the new state
     __shared__ double sRed[32];
     const int tid = threadIdx.x;
-    for (int t = tid; t < S::NOPS; t += blockDim.x) sOps[t] = a.ops[t];
+    S::fill(sOps, a.ops);
     pdl_launch_dependents();
     pdl_wait();   // the state and traces come from the previous launches
     const int el = tid / TPE, k = tid - el * TPE;
@@ -259,8 +275,11 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
     const int edge = k / N1, fp = k - edge * N1;
     const T g = T(a.gamma);
     constexpr bool kRef = UsesRef<T>::value;
+    const T* Tin = after_wait(a.Tin);
+    const T* FV = after_wait(a.FV);
 
-    // ---- A1: loads
+    // ---- A1: loads; the stage state (NS) and face jumps into shared memory;
+    // the common flux of the flux points
     T ue[4] = {T(0), T(0), T(0), T(0)};
     if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
@@ -269,23 +288,8 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
     if (is_fp) {
         r = a.edges[e * 4 + edge];
         load_normal(a.enrm + e * 4 + edge, nr);
-        load4_nc(a.Tin + (e * 4 * N1 + k) * 4, qo);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) qn[v] = qo[v];
-        if (!(r.flags & kEdgeOrphan)) load4_nc(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
-        if constexpr (VISC) {
-            load4_nc(a.FV + (e * 4 * N1 + k) * 4, fv);
-            if (!(r.flags & (kEdgeOrphan | kEdgeBoundary))) {
-                T fn[4];
-                load4_nc(a.FV + (((long long)r.nbr * 4 + r.nbr_edge) * N1 + (N1 - 1 - fp)) * 4, fn);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) fv[v] += fn[v];
-            }
-            T d[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) d[v] = (r.flags & kEdgeOrphan) ? T(0) : T(0.5) * (qn[v] - qo[v]);
-            store4(sD + el * DS + k * 4, d);
-        }
+        load4_nc(Tin + (e * 4 * N1 + k) * 4, qo);
+        if constexpr (VISC) load4_nc(FV + (e * 4 * N1 + k) * 4, fv);
     }
     T u[4], ji[4], Jd = T(1);
     if (is_sp) {
@@ -302,9 +306,44 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
 #pragma unroll
                 for (int v = 0; v < 4; ++v) w[v] = u[v];
             }
-#pragma unroll
-            for (int v = 0; v < 4; ++v) sU[el * ES + v * FS + k] = w[v];
+            store4(sU + el * ES + 4 * k, w);
         }
+    }
+    const bool face = is_fp && !(r.flags & kEdgeOrphan);
+    if (face) {
+        load4_nc(Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
+        if (VISC && !(r.flags & kEdgeBoundary)) {
+            T fn[4];
+            load4_nc(FV + (((long long)r.nbr * 4 + r.nbr_edge) * N1 + (N1 - 1 - fp)) * 4, fn);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) fv[v] += fn[v];
+        }
+    }
+    if constexpr (VISC) {
+        if (is_fp) {
+            T d[4];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) d[v] = face ? T(0.5) * (qn[v] - qo[v]) : T(0);
+            store4(sD + el * DS + k * 4, d);
+        }
+    }
+    T Fd[4] = {T(0), T(0), T(0), T(0)};
+    if (face) {
+        const bool right = (r.flags & kEdgeRight) != 0;
+        T UL[4], UR[4], Fc[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) { UL[v] = right ? qn[v] : qo[v]; UR[v] = right ? qo[v] : qn[v]; }
+        riemann<RIEM>(UL, UR, nr[0], nr[1], g, Fc);
+        if constexpr (kRef) {
+            T Fe[4];
+            ref_flux_n(ue, g, nr[0], nr[1], Fe);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
+        }
+        const T sf = nr[2] * T(1.0 / tri_ref_len(edge));
+        const T ss = right ? -sf : sf;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Fd[v] = ss * (Fc[v] - fv[v]);
     }
     if constexpr (VISC) __syncthreads();
 
@@ -320,49 +359,32 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
         }
         if constexpr (VISC) {
             T Qx[4], Qy[4], Fv[4], Gv[4];
-            tri_gradient<NT, NFT, FS>(sU + el * ES, sD + el * DS, sOps + Lo::DR, sOps + Lo::DSo, sOps + Lo::PHI,
-                                      k, ji, Qx, Qy);
+            tri_gradient<P>(sU + el * ES, sD + el * DS, sOps, k, ji, Qx, Qy);
             viscous_flux_f(u, rcp_any(u[0]), Qx, Qy, g, inv_reynolds(a), T(a.kfac), Fv, Gv);
 #pragma unroll
             for (int v = 0; v < 4; ++v) { F[v] -= Fv[v]; G[v] -= Gv[v]; }
         }
+        T ft[4], gt[4];
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
-            sF[el * ES + v * FS + k] = Jd * (ji[0] * F[v] + ji[1] * G[v]);
-            sG[el * ES + v * FS + k] = Jd * (ji[2] * F[v] + ji[3] * G[v]);
+            ft[v] = Jd * (ji[0] * F[v] + ji[1] * G[v]);
+            gt[v] = Jd * (ji[2] * F[v] + ji[3] * G[v]);
         }
+        store4(sF + el * ES + 4 * k, ft);
+        store4(sG + el * ES + 4 * k, gt);
     }
     __syncthreads();
 
-    // ---- B: interface terms
+    // ---- B: flux differences at the faces (NS: the jumps were consumed in A2)
     if (is_fp) {
-        T Fd[4] = {T(0), T(0), T(0), T(0)};
-        if (!(r.flags & kEdgeOrphan)) {
-            const bool right = (r.flags & kEdgeRight) != 0;
-            T UL[4], UR[4], Fc[4];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) { UL[v] = right ? qn[v] : qo[v]; UR[v] = right ? qo[v] : qn[v]; }
-            riemann<RIEM>(UL, UR, nr[0], nr[1], g, Fc);
-            if constexpr (kRef) {
-                T Fe[4];
-                ref_flux_n(ue, g, nr[0], nr[1], Fe);
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v];
-            }
-            if constexpr (VISC) {
-#pragma unroll
-                for (int v = 0; v < 4; ++v) Fc[v] -= fv[v];
-            }
-            const T sf = nr[2] * T(1.0 / tri_ref_len(edge));
-            const T ss = right ? -sf : sf;
-            T fx[4], gy[4];
-            tri_interp<NT, FS>(sF + el * ES, sOps + Lo::L + k * NT, fx);
-            tri_interp<NT, FS>(sG + el * ES, sOps + Lo::L + k * NT, gy);
-            const T nx = T(tri_nref_x(edge)), ny = T(tri_nref_y(edge));
-#pragma unroll
-            for (int v = 0; v < 4; ++v) Fd[v] = ss * Fc[v] - (fx[v] * nx + gy[v] * ny);
+        if (face) {
+            const T* Lr = sOps + S::LO + k * S::RL;
+            V4<T> acc = v4(Fd);
+            acc = v4_fma(weight<T>(T(-tri_nref_x(edge))), tri_dot<NT>(sF + el * ES, Lr), acc);
+            acc = v4_fma(weight<T>(T(-tri_nref_y(edge))), tri_dot<NT>(sG + el * ES, Lr), acc);
+            v4_get(acc, Fd);
         }
-        store4(sD + el * DS + k * 4, Fd);   // (NS: the jumps were consumed in A2)
+        store4(sD + el * DS + k * 4, Fd);
     }
     __syncthreads();
 
@@ -372,29 +394,19 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
         const long long idx = e * NSP + k;
         double u0[4];
         if (a.stage >= 2) gload4(a.U0 + idx * 4, u0);
-        T div[4] = {T(0), T(0), T(0), T(0)};
-        const T* Dr = sOps + Lo::DR + k * NT;
-        const T* Dsr = sOps + Lo::DSo + k * NT;
+        V4<T> div = tri_dot<NFT>(sD + el * DS, sOps + S::PHI + k * S::RF);
 #pragma unroll
         for (int m = 0; m < NT; ++m) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                div[v] = fma_any(Dr[m], sF[el * ES + v * FS + m], div[v]);
-                div[v] = fma_any(Dsr[m], sG[el * ES + v * FS + m], div[v]);
-            }
-        }
-        const T* Ph = sOps + Lo::PHI + k * NFT;
-#pragma unroll
-        for (int q = 0; q < NFT; ++q) {
-            T d[4];
-            load4(sD + el * DS + q * 4, d);
-#pragma unroll
-            for (int v = 0; v < 4; ++v) div[v] = fma_any(Ph[q], d[v], div[v]);
+            T x, y;
+            load_pair(sOps + k * S::RD + 2 * m, x, y);
+            div = v4_fma(weight<T>(x), v4_load(sF + el * ES + 4 * m), div);
+            div = v4_fma(weight<T>(y), v4_load(sG + el * ES + 4 * m), div);
         }
         const T iJ = rcp_any(Jd);
         T res[4];
+        v4_get(div, res);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) res[v] = -div[v] * iJ;
+        for (int v = 0; v < 4; ++v) res[v] = -res[v] * iJ;
         if (a.stage == 0) {
             store_residual(a, idx, res, rsq);
         } else {
@@ -409,8 +421,7 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
 #pragma unroll
                 for (int v = 0; v < 4; ++v) un[v] = T(uo[v]);
             }
-#pragma unroll
-            for (int v = 0; v < 4; ++v) sU[el * ES + v * FS + k] = un[v];
+            store4(sU + el * ES + 4 * k, un);
             if (a.stage == 3) {
 #pragma unroll
                 for (int v = 0; v < 4; ++v) rsq += double(res[v]) * double(res[v]);
@@ -427,7 +438,7 @@ k_tri_stage(const StageArgsT<T> a, const int32_t* __restrict__ elist, long long 
     // ---- D: traces of the new state and ghost rows
     if (is_fp) {
         T t[4];
-        tri_interp<NT, FS>(sU + el * ES, sOps + Lo::L + k * NT, t);
+        v4_get(tri_dot<NT>(sU + el * ES, sOps + S::LO + k * S::RL), t);
         if constexpr (kRef) {
 #pragma unroll
             for (int v = 0; v < 4; ++v) t[v] += ue[v];
