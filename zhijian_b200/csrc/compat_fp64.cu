@@ -484,11 +484,11 @@ cudaError_t launch_stage_t(const StageArgs& a, cudaStream_t s, int* grid_out) {
     const long long grid = (a.n_elem + S::EB - 1) / S::EB;
     if (grid_out) *grid_out = (int)grid;
     if (grid <= 0) return cudaSuccess;
-    // Prefer the largest shared-memory carveout so kMinBlocks CTAs fit per SM.
     static bool carveout_set = false;
     if (!carveout_set) {
-        cudaFuncSetAttribute(k_compat_stage<P>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             cudaSharedmemCarveoutMaxShared);
+        constexpr size_t smem = sizeof(double) * (OpTable<P + 1, double>::N + 32 +
+                                                  S::EB * (3 * Tiles<P, double>::FP + Tiles<P, double>::DP));
+        set_carveout(k_compat_stage<P>, carveout_percent(carveout_bytes(kMinBlocks, smem)));
         carveout_set = true;
     }
     return launch_programmatic(k_compat_stage<P>, (unsigned)grid, S::THREADS, s, a);

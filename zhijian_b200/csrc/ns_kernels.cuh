@@ -57,6 +57,13 @@
 #ifndef ZJ_NSG32_MIN_BLOCKS
 #define ZJ_NSG32_MIN_BLOCKS 12    // mixed-precision point-per-thread gradient kernel
 #endif
+// Threads per CTA of the gradient kernel by lines (rounded down to whole
+// elements): 64 spread a coarse mesh over more SMs and interleave more phases;
+// against 128 per step 20 x 20 P3 FP32 -1.4 %, 64 x 64 and 256 x 256 FP64
+// -0.6 and -0.8 %, P5 FP32 -0.5 %; 32 cost P5 4 %.
+#ifndef ZJ_LINE_THREADS
+#define ZJ_LINE_THREADS 64
+#endif
 #ifndef ZJ_NSL_MIN_BLOCKS
 #define ZJ_NSL_MIN_BLOCKS 4       // FP64 gradient kernel by lines (128 registers)
 #endif
@@ -257,7 +264,7 @@ k_ns_grad(const StageArgsT<T> a) {
 template <int P, typename T>
 struct LineShape {
     static constexpr int N1 = P + 1, NSP = N1 * N1, NFT = 4 * N1;
-    static constexpr int EB = kCtaThreads / (2 * N1);   // elements per CTA
+    static constexpr int EB = ZJ_LINE_THREADS / (2 * N1);   // elements per CTA
     static constexpr int THREADS = EB * 2 * N1;
     static constexpr int NOPS = N1 * N1 + 4 * N1;
     // derivative tile: [el][role][var][a*R + b]
@@ -283,7 +290,7 @@ struct LineShape {
     static constexpr int MIN_BLOCKS_128 =
         sizeof(T) == 8 ? ZJ_NSL_MIN_BLOCKS
                        : (P <= 3 ? ZJ_NSL32_MIN_BLOCKS : ZJ_NSL32_MIN_BLOCKS_HI);
-    static constexpr int MIN_BLOCKS = MIN_BLOCKS_128 * 128 / kCtaThreads > 0 ? MIN_BLOCKS_128 * 128 / kCtaThreads : 1;
+    static constexpr int MIN_BLOCKS = MIN_BLOCKS_128 * 128 / ZJ_LINE_THREADS > 0 ? MIN_BLOCKS_128 * 128 / ZJ_LINE_THREADS : 1;
 };
 
 // 16-byte asynchronous global -> shared copy (cp.async, cached in L2 only),
@@ -652,6 +659,17 @@ k_ns_stage(const StageArgsT<T> a) {
     }
 }
 
+// One split for the gradient and the stage kernel.
+template <int P, typename T>
+constexpr int ns_carveout() {
+    const int st = carveout_bytes(NSMinBlocks<T, P>::stage, stage_smem<P, T>());
+    if constexpr (IsDual<T>::value) return 100;
+    else {
+        const int gr = carveout_bytes(LineShape<P, T>::MIN_BLOCKS, LineShape<P, T>::SMEM);
+        return carveout_percent(st > gr ? st : gr);
+    }
+}
+
 template <int P, typename T>
 cudaError_t ns_grad_t(const StageArgsT<T>& a, cudaStream_t s) {
     if constexpr (!IsDual<T>::value) {
@@ -660,7 +678,7 @@ cudaError_t ns_grad_t(const StageArgsT<T>& a, cudaStream_t s) {
         if (grid <= 0) return cudaSuccess;
         static bool set = false;
         if (!set) {
-            prefer_shared(k_ns_grad_lines<P, T>);
+            set_carveout(k_ns_grad_lines<P, T>, ns_carveout<P, T>());
             cudaFuncSetAttribute(k_ns_grad_lines<P, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM);
             set = true;
         }
@@ -670,7 +688,7 @@ cudaError_t ns_grad_t(const StageArgsT<T>& a, cudaStream_t s) {
         const long long grid = ((a.elist ? a.n_list : a.n_elem) + S::EB - 1) / S::EB;
         if (grid <= 0) return cudaSuccess;
         static bool set = false;
-        if (!set) { prefer_shared(k_ns_grad<P, T>); set = true; }
+        if (!set) { set_carveout(k_ns_grad<P, T>, ns_carveout<P, T>()); set = true; }
         return launch_programmatic(k_ns_grad<P, T>, (unsigned)grid, S::THREADS, s, a);
     }
 }
@@ -681,7 +699,7 @@ cudaError_t ns_stage_t(const StageArgsT<T>& a, cudaStream_t s) {
     const long long grid = ((a.elist ? a.n_list : a.n_elem) + S::EB - 1) / S::EB;
     if (grid <= 0) return cudaSuccess;
     static bool set = false;
-    if (!set) { prefer_shared(k_ns_stage<P, RIEM, T>); set = true; }
+    if (!set) { set_carveout(k_ns_stage<P, RIEM, T>, ns_carveout<P, T>()); set = true; }
     return launch_programmatic(k_ns_stage<P, RIEM, T>, (unsigned)grid, S::THREADS, s, a);
 }
 

@@ -417,10 +417,16 @@ k_phys_traces(const StageArgsT<T> a) {
     }
 }
 
-template <class K>
-void prefer_shared(K kernel) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         cudaSharedmemCarveoutMaxShared);
+// Shared memory of a stage kernel's CTA: operators, four tiles, reductions.
+template <int P, typename T>
+constexpr size_t stage_smem() {
+    using S = Shape<P, EbDiv<T>::value>;
+    return sizeof(Weight<T>) * OpTable<P + 1, T>::N +
+           sizeof(T) * S::EB * (3 * Tiles<P, T>::FP + Tiles<P, T>::DP) + 32 * sizeof(double);
+}
+template <int P, typename T>
+constexpr int phys_carveout() {
+    return carveout_percent(carveout_bytes(PhysMinBlocks<T>::value, stage_smem<P, T>()));
 }
 
 template <int P, int RIEM, typename T>
@@ -429,7 +435,7 @@ cudaError_t phys_stage_t(const StageArgsT<T>& a, cudaStream_t s) {
     const long long grid = ((a.elist ? a.n_list : a.n_elem) + S::EB - 1) / S::EB;
     if (grid <= 0) return cudaSuccess;
     static bool carveout_set = false;
-    if (!carveout_set) { prefer_shared(k_phys_stage<P, RIEM, T>); carveout_set = true; }
+    if (!carveout_set) { set_carveout(k_phys_stage<P, RIEM, T>, phys_carveout<P, T>()); carveout_set = true; }
     return launch_programmatic(k_phys_stage<P, RIEM, T>, (unsigned)grid, S::THREADS, s, a);
 }
 

@@ -462,6 +462,8 @@ cudaError_t tri_grad_t(const StageArgsT<T>& a, const int32_t* elist, long long n
     using S = TriShape<P, T>;
     const long long grid = (n + S::EB - 1) / S::EB;
     if (grid <= 0) return cudaSuccess;
+    static bool set = false;
+    if (!set) { set_carveout(k_tri_grad<P, T>, ns_carveout<P, T>()); set = true; }   // the quads' split
     return launch_programmatic(k_tri_grad<P, T>, (unsigned)grid, S::THREADS, s, a, elist, n);
 }
 
@@ -470,6 +472,11 @@ cudaError_t tri_stage_t(const StageArgsT<T>& a, const int32_t* elist, long long 
     using S = TriShape<P, T>;
     const long long grid = (n + S::EB - 1) / S::EB;
     if (grid <= 0) return cudaSuccess;
+    static bool set = false;
+    if (!set) {   // the quads' split
+        set_carveout(k_tri_stage<P, RIEM, VISC, T>, VISC ? ns_carveout<P, T>() : phys_carveout<P, T>());
+        set = true;
+    }
     return launch_programmatic(k_tri_stage<P, RIEM, VISC, T>, (unsigned)grid, S::THREADS, s, a, elist, n);
 }
 
