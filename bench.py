@@ -82,11 +82,11 @@ def algorithmic_bytes_per_element(p, w_s=8, w_g=8, w_t=8, viscous=False):
     """Bytes one element moves per residual evaluation with the fused RK stage:
     w_s*12*n_sp (stage state, base state, output) + w_g*5*n_sp (J and four
     metric terms) + w_t*32*n_f (own trace write + neighbour trace read)
-    [+ w_t*64*n_f for the gradient traces of Navier-Stokes]."""
+    [+ w_t*32*n_f for the viscous shares of Navier-Stokes, likewise]."""
     nsp, nf = (p + 1) ** 2, p + 1
     b = w_s * 12 * nsp + w_g * 5 * nsp + w_t * 32 * nf
     if viscous:
-        b += w_t * 64 * nf
+        b += w_t * 32 * nf
     return b
 
 
