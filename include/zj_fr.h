@@ -332,7 +332,9 @@ zj_status zj_step_vjp(zj_solver* s, const double* U_dev, double dt, const double
  * G_dev holds dJ/dU(final) on entry and dJ/dU(initial) on return.  Optional
  * outputs: *dRe = dJ/dRe, *bytes = device bytes the checkpoints and segment
  * states took, *ms_forward / *ms_adjoint = device times of the checkpointed
- * forward sweep and of the backward sweep (CUDA events). */
+ * forward sweep and of the backward sweep (CUDA events).  The handle keeps
+ * that block for its next call if it is at most 1 GiB (freed with the handle);
+ * a larger one is freed before the call returns. */
 zj_status zj_adjoint_run(zj_solver* s, double dt, int nsteps, int k_ckpt, double* G_dev,
                          double* dRe, int64_t* bytes, double* ms_forward, double* ms_adjoint);
 

@@ -245,16 +245,14 @@ k_ns_grad(const StageArgsT<T> a) {
 // (0..N1-1, j)) and one per column i (an eta-line (i, 0..N1-1)).  The CTA
 // first stages its elements' states into shared memory with 16-byte cp.async
 // copies (each 16-byte piece fetched once), while every line thread loads the
-// traces at its line's two end points (its own and the neighbour's).  A line thread then takes the corrected derivative along its
-// line in registers (row: dU/dxi with the jumps of edges 1 and 3; column:
+// traces at its line's two end points (its own and the neighbour's).  A line
+// thread then takes the corrected derivative along its line in registers (row: dU/dxi with the jumps of edges 1 and 3; column:
 // dU/deta with those of edges 0 and 2) and swaps derivatives with the
 // crossing lines through one shared tile.  It forms Q = (xi_x dU/dxi + eta_x
 // dU/deta, xi_y dU/dxi + eta_y dU/deta) at its N1 points and the traces of Q
 // at its two end points (row j: edge 1 point j with l(+1), edge 3 point
 // N1-1-j with l(-1); column i: edge 0 point i with l(-1), edge 2 point
-// N1-1-i with l(+1)).  Every sum is corrected_gradient_tr's and
-// trace_point's, term for term in the same order, so the traces equal
-// k_ns_grad's.
+// N1-1-i with l(+1)), and from them the element's viscous shares.
 //
 // Rows and columns run the same instruction stream (the role only selects
 // strides, edges and weights) and fill separate warps at P3.  The derivative

@@ -35,7 +35,8 @@ struct Shape {
     static constexpr int EB = (kCtaThreads / TPE / EBDIV) > 0 ? (kCtaThreads / TPE / EBDIV) : 1;
     static constexpr int THREADS = EB * TPE;
     static constexpr int NOPS = N1 * N1 + 4 * N1;
-    // Shared-memory layout of per-element fields (doubles): [var][eta row][xi]
+    // Shared-memory layout of per-element fields kept a variable at a time
+    // (the transposed kernels' doubles): [var][eta row][xi]
     // with rows padded to an even length so every row starts 16-byte aligned
     // (vector loads), and a per-element stride of 6 mod 16 so the elements
     // that share a warp start on different banks.  Flux differences use
