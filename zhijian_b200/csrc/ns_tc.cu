@@ -149,12 +149,13 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
     float fv[4] = {0.f, 0.f, 0.f, 0.f};   // common normal viscous flux: both sides' shares
     if (is_fp) {
         const float* Tin = after_wait(a.Tin);
+        const float* FV = after_wait(a.FV);
         load_own_face<N1>(a, Tin, e, edge, fp, f);
         load_neighbour_face<N1>(a, Tin, fp, f);
-        load4_nc(a.FV + (e * NFT + k) * 4, fv);
+        load4_nc(FV + (e * NFT + k) * 4, fv);
         if (has_neighbour_gradient(f.r)) {
             float fn[4];
-            load4_nc(a.FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
+            load4_nc(FV + (neighbour_row(f.r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, fn);
 #pragma unroll
             for (int v = 0; v < 4; ++v) fv[v] += fn[v];
         }
