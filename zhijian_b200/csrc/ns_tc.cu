@@ -247,7 +247,7 @@ k_ns_stage_tc(const StageArgsT<float> a, const __grid_constant__ CUtensorMap ama
         float Fe[4];
         ref_flux_n(ue, g, f.nx, f.ny, Fe);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) Fc[v] -= Fe[v] + fv[v];
+        for (int v = 0; v < 4; ++v) Fc[v] = (Fc[v] - Fe[v]) - fv[v];   // Fe + fv would round fv at the size of Fe
     }
 
     // ---- the product: tensor memory -> the result tile (rows 16q..16q+15 sit
