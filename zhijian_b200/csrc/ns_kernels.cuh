@@ -660,9 +660,9 @@ k_ns_stage(const StageArgsT<T> a) {
 // One split for the gradient and the stage kernel.
 template <int P, typename T>
 constexpr int ns_carveout() {
-    const int st = carveout_bytes(NSMinBlocks<T, P>::stage, stage_smem<P, T>());
-    if constexpr (IsDual<T>::value) return 100;
+    if constexpr (IsDual<T>::value) return 100;   // as phys_carveout
     else {
+        const int st = carveout_bytes(NSMinBlocks<T, P>::stage, stage_smem<P, T>());
         const int gr = carveout_bytes(LineShape<P, T>::MIN_BLOCKS, LineShape<P, T>::SMEM);
         return carveout_percent(st > gr ? st : gr);
     }

@@ -424,9 +424,13 @@ constexpr size_t stage_smem() {
     return sizeof(Weight<T>) * OpTable<P + 1, T>::N +
            sizeof(T) * S::EB * (3 * Tiles<P, T>::FP + Tiles<P, T>::DP) + 32 * sizeof(double);
 }
+// (Dual numbers have no launch bound that says how many CTAs are resident, so
+// they take the largest split: sized for one CTA, J V and J^T J V on 160 x 157 Euler
+// quads, P3, Roe, took 430 us instead of 128.)
 template <int P, typename T>
 constexpr int phys_carveout() {
-    return carveout_percent(carveout_bytes(PhysMinBlocks<T>::value, stage_smem<P, T>()));
+    if constexpr (IsDual<T>::value) return 100;
+    else return carveout_percent(carveout_bytes(PhysMinBlocks<T>::value, stage_smem<P, T>()));
 }
 
 template <int P, int RIEM, typename T>
