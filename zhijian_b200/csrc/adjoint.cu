@@ -279,7 +279,7 @@ k_adj_ns(const AdjArgs a) {
     const bool is_sp = valid && k < NSP, is_fp = valid && k < NFT;
     const int edge = k / N1, fp = k - edge * N1;
     const int i = k % N1, j = k / N1;
-    const double g = a.gamma, iRe = a.iRe, kfac = a.kfac;
+    const double g = a.gamma, Re = a.Re, Pr = a.Pr;
 
     // ---- 1: loads
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
@@ -342,7 +342,7 @@ k_adj_ns(const AdjArgs a) {
             mGb[v] = -Gb[v];
         }
         adj::euler_flux_vjp(u, g, Fb, Gb, ub);
-        re_acc -= adj::viscous_vjp(u, Qx, Qy, g, iRe, kfac, mFb, mGb, ub, Qxb, Qyb) * iRe;
+        re_acc -= adj::viscous_vjp(u, Qx, Qy, g, Re, Pr, mFb, mGb, ub, Qxb, Qyb) / Re;
     }
     double tb[4] = {0.0, 0.0, 0.0, 0.0};
     if (is_fp) {
@@ -373,8 +373,8 @@ k_adj_ns(const AdjArgs a) {
                 Fvb[v] = -Fnb[v] * nx;
                 Gvb[v] = -Fnb[v] * ny;
             }
-            const double dv = adj::viscous_vjp(Ua, dxa, dya, g, iRe, kfac, Fvb, Gvb, Uab, dxb, dyb);
-            if (!right) re_acc -= dv * iRe;   // once per face: on its left element
+            const double dv = adj::viscous_vjp(Ua, dxa, dya, g, Re, Pr, Fvb, Gvb, Uab, dxb, dyb);
+            if (!right) re_acc -= dv / Re;   // once per face: on its left element
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 ULb[v] += 0.5 * Uab[v];

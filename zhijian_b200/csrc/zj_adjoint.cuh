@@ -57,11 +57,10 @@ __device__ __forceinline__ void euler_flux_vjp(const double* s, double g, const 
 // Reverse sweep of phys::viscous_flux: given Fvb, Gvb (components 1..3; the
 // mass components of the viscous flux are zero), adds the adjoints of the
 // state s and of the gradients dx = dU/dx, dy = dU/dy into sb, dxb, dyb.
-// iRe = 1/Re, kfac = gamma/((gamma-1) Pr).  Returns Fvb . Fv + Gvb . Gv: the
-// viscous flux is proportional to 1/Re, so minus this over Re is the flux
-// adjoint's Reynolds-number derivative.
+// Returns Fvb . Fv + Gvb . Gv: the viscous flux is proportional to 1/Re, so
+// minus this over Re is the flux adjoint's Reynolds-number derivative.
 __device__ __forceinline__ double viscous_vjp(const double* s, const double* dx, const double* dy,
-                                            double g, double iRe, double kfac, const double* Fvb,
+                                            double g, double Re, double Pr, const double* Fvb,
                                             const double* Gvb, double* sb, double* dxb,
                                             double* dyb) {
     // forward recomputation (the operations of phys::viscous_flux)
@@ -76,8 +75,8 @@ __device__ __forceinline__ double viscous_vjp(const double* s, const double* dx,
     const double dpdx = c * (dx[3] - 0.5 * dx[0] * q2 - s[0] * (u * dudx + v * dvdx));
     const double dpdy = c * (dy[3] - 0.5 * dy[0] * q2 - s[0] * (u * dudy + v * dvdy));
     const double dTdx = (dpdx - Tm * dx[0]) * ir, dTdy = (dpdy - Tm * dy[0]) * ir;
-    const double mu = zj_pow07(Tm) * iRe;
-    const double kc = kfac;
+    const double mu = zj_pow07(Tm) / Re;
+    const double kc = g / (c * Pr);
     const double k = mu * kc;
     const double div = dudx + dvdy, lam = (-2.0 / 3.0) * mu;
     const double txx = 2.0 * mu * dudx + lam * div, tyy = 2.0 * mu * dvdy + lam * div;
@@ -98,7 +97,7 @@ __device__ __forceinline__ double viscous_vjp(const double* s, const double* dx,
     mub += lamb * (-2.0 / 3.0);
     dudxb += divb; dvdyb += divb;
     mub += kb * kc;
-    double Tmb = (Tm != 0.0) ? mub * 0.7 * mu * rcp_any(Tm) : 0.0;
+    double Tmb = (Tm != 0.0) ? mub * 0.7 * mu / Tm : 0.0;
     double irb = 0.0;
     double dpdxb = dTdxb * ir, dpdyb = dTdyb * ir;
     Tmb -= dTdxb * dx[0] * ir + dTdyb * dy[0] * ir;
@@ -249,11 +248,8 @@ __device__ __forceinline__ void roe_vjp(const double* UL, const double* UR, doub
     double uLb = -dub, uRb = dub, vLb = -dvb, vRb = dvb, rhoLb = -drhob, rhoRb = drhob;
     // entropy fix: l = (lo^2 + eps^2) / (2 eps)
     double epsb = 0.0, l1ob = l1b, l4ob = l4b;
-    if (fix1 || fix4) {
-        const double ie = rcp_any(eps);
-        if (fix4) { l4ob = l4b * l4o * ie; epsb += l4b * (0.5 - 0.5 * (l4o * ie) * (l4o * ie)); }
-        if (fix1) { l1ob = l1b * l1o * ie; epsb += l1b * (0.5 - 0.5 * (l1o * ie) * (l1o * ie)); }
-    }
+    if (fix4) { l4ob = l4b * l4o / eps; epsb += l4b * (0.5 - l4o * l4o / (2.0 * eps * eps)); }
+    if (fix1) { l1ob = l1b * l1o / eps; epsb += l1b * (0.5 - l1o * l1o / (2.0 * eps * eps)); }
     cb += 0.1 * epsb;
     const double s4 = (vnRoe + c < 0.0) ? -1.0 : 1.0;
     const double s2 = (vnRoe < 0.0) ? -1.0 : 1.0;
@@ -262,7 +258,7 @@ __device__ __forceinline__ void roe_vjp(const double* UL, const double* UR, doub
     cb += l4ob * s4 - l1ob * s1;
     // c = sqrt(max(carg, 1e-10))
     if (carg >= 1e-10 && c > 0.0) {
-        const double cargb = cb * 0.5 * rcp_any(c);
+        const double cargb = cb * 0.5 / c;
         HRoeb += cargb * (g - 1.0);
         qsqb -= cargb * (g - 1.0) * 0.5;
     }
@@ -277,8 +273,8 @@ __device__ __forceinline__ void roe_vjp(const double* UL, const double* UR, doub
     const double idenb = uRoeb * (sL * uL + sR * uR) + vRoeb * (sL * vL + sR * vR) + HRoeb * (sL * HL + sR * HR);
     sLb += rhoRoeb * sR; sRb += rhoRoeb * sL;
     if (ssum >= 1e-10) { const double t = -idenb * iden * iden; sLb += t; sRb += t; }
-    if (sL > 0.0) rhoLb += sLb * 0.5 * rcp_any(sL);
-    if (sR > 0.0) rhoRb += sRb * 0.5 * rcp_any(sR);
+    if (sL > 0.0) rhoLb += sLb * 0.5 / sL;
+    if (sR > 0.0) rhoRb += sRb * 0.5 / sR;
     // H = (U3 + p) ir
     ULb[3] += HLb * irL; pLb += HLb * irL; double irLb = HLb * (UL[3] + pL);
     URb[3] += HRb * irR; pRb += HRb * irR; double irRb = HRb * (UR[3] + pR);
