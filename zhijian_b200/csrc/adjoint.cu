@@ -30,14 +30,6 @@
 #include "ns_kernels.cuh"
 #include "zj_adjoint.cuh"
 
-// Navier-Stokes adjoint kernel: 250 registers and 4 CTAs of 64 threads per SM,
-// no spills.  168 registers and 6 CTAs spill 500 bytes; on 91 x 57 quads (P2, one
-// wave) a Gauss-Newton product then takes 97 us instead of 87, on 128 x 128
-// (P3) eight adjoint steps 3.46 ms instead of 3.48.
-#ifndef ZJ_ADJ_MIN_BLOCKS
-#define ZJ_ADJ_MIN_BLOCKS 2
-#endif
-
 namespace zj {
 namespace {
 
@@ -171,8 +163,11 @@ k_adj_dfbar(const AdjArgs a) {
 }
 
 // ---------------------------------------------------------- pass B, Euler --
+// CTAs of 128 threads per SM: 2 (about 245 registers, no spills); at P3 3, at
+// 168 registers (160 x 157, P3: Rusanov 194 -> 163 us, Roe 66 -> 56; 40 x 37,
+// under a wave: 27 -> 29).
 template <int P, int RIEM>
-__global__ void __launch_bounds__(Shape<P>::THREADS)
+__global__ void __launch_bounds__(Shape<P>::THREADS, P == 3 ? 3 : 2)
 k_adj_euler(const AdjArgs a) {
     using S = Shape<P>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
@@ -255,8 +250,17 @@ k_adj_euler(const AdjArgs a) {
 }
 
 // ---------------------------------------------------- pass B, Navier-Stokes --
+// Up to P3 4 CTAs of 60 to 64 threads per SM (about 250 registers, no spills) with
+// the ghost state's transpose as a call; from P4 up 6 CTAs (168 registers,
+// spills of 0.3 to 0.4 KB) with the transpose inlined, as these CTAs' 50 or 36
+// threads leave their warps partly empty. Transposed residual, the first form
+// against the second: P3 HLLC 50 and 57 us on 40 x 37, P1 Rusanov 62 and 70 on
+// 90 x 87; P4 HLLC 79 and 69 on 40 x 37, P5 Roe 455 and 416 on 160 x 157.
+template <int P> constexpr bool kGhostCall = P <= 3;
+template <int P> constexpr int kAdjNsBlocks = P <= 3 ? 4 : 6;
+
 template <int P, int RIEM>
-__global__ void __launch_bounds__(Shape<P, 2>::THREADS, ZJ_ADJ_MIN_BLOCKS * kCtaScale)
+__global__ void __launch_bounds__(Shape<P, 2>::THREADS, kAdjNsBlocks<P>)
 k_adj_ns(const AdjArgs a) {
     using S = Shape<P, 2>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
@@ -386,7 +390,7 @@ k_adj_ns(const AdjArgs a) {
                 tb[v] = right ? URb[v] : ULb[v];
             }
             if (bnd)
-                adj::ghost_vjp(qo, nx, ny, edge_bc_type(r.flags), a.bc + (long long)r.nbr_edge * 8, g,
+                adj::ghost_vjp_of<kGhostCall<P>>(qo, nx, ny, edge_bc_type(r.flags), a.bc + (long long)r.nbr_edge * 8, g,
                                URb, tb);
         }
         store4(sTQ + el * 2 * DS + k * 8, tq);
@@ -446,7 +450,7 @@ k_adj_ns(const AdjArgs a) {
             double hb[4];
 #pragma unroll
             for (int v = 0; v < 4; ++v) hb[v] = 0.5 * dub[v];
-            adj::ghost_vjp(qo, nx, ny, edge_bc_type(r.flags), a.bc + (long long)r.nbr_edge * 8, g,
+            adj::ghost_vjp_of<kGhostCall<P>>(qo, nx, ny, edge_bc_type(r.flags), a.bc + (long long)r.nbr_edge * 8, g,
                            hb, tb);
         }
         gstore4(a.Tb + (e * NFT + k) * 4, tb);

@@ -308,20 +308,35 @@ __device__ __forceinline__ void riemann_vjp(const double* UL, const double* UR, 
         }
         phys::riemann<RIEM>(L, R, Dual(nx), Dual(ny), Dual(g), F);
         const double t = Fb[0] * F[0].d + Fb[1] * F[1].d + Fb[2] * F[2].d + Fb[3] * F[3].d;
-        // (selected, not indexed: an index would put the arrays in local memory)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            ULb[v] += (k == v) ? t : 0.0;
-            URb[v] += (k == 4 + v) ? t : 0.0;
-        }
+        if (k < 4) ULb[k] += t;
+        else URb[k - 4] += t;
     }
     }
 }
 
-// (dGhost/dUi)^T Gb: four tangent evaluations of the ghost state on dual
-// numbers.  A call, not inlined: boundary faces are few, and inlined twice
-// its code and registers (every boundary class on duals) burdened every
-// thread of the adjoint kernels.
+// (dGhost/dUi)^T Gb into Uib (accumulated): four tangent evaluations of the
+// ghost state on dual numbers.
+__device__ __forceinline__ void ghost_vjp(const double* Ui, double nx, double ny, int bct,
+                                          const double* bcd, double g, const double* Gb,
+                                          double* Uib) {
+    Dual bd[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) bd[i] = Dual(bcd[i]);
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        Dual Ud[4], Gd[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Ud[v] = Dual(Ui[v], (k == v) ? 1.0 : 0.0);
+        phys::ghost_phys(Ud, Dual(nx), Dual(ny), bct, bd, Dual(g), Gd);
+        const double t = Gb[0] * Gd[0].d + Gb[1] * Gd[1].d + Gb[2] * Gd[2].d + Gb[3] * Gd[3].d;
+        // (selected, not indexed: an index would put the array in local memory)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Uib[v] = (k == v) ? Uib[v] + t : Uib[v];
+    }
+}
+
+// The same as a call: boundary faces are few, and inlined its code and
+// registers (every boundary class on duals) burden every thread of a kernel.
 __device__ __noinline__ double4 ghost_vjp_call(double4 Ui, double nx, double ny, int bct, const double* bcd,
                                                double g, double4 Gb) {
     Dual bd[8];
@@ -338,14 +353,16 @@ __device__ __noinline__ double4 ghost_vjp_call(double4 Ui, double nx, double ny,
     }
     return make_double4(r[0], r[1], r[2], r[3]);
 }
-
-// The same added to Uib.
-__device__ __forceinline__ void ghost_vjp(const double* Ui, double nx, double ny, int bct,
-                                          const double* bcd, double g, const double* Gb,
-                                          double* Uib) {
-    const double4 r = ghost_vjp_call(make_double4(Ui[0], Ui[1], Ui[2], Ui[3]), nx, ny, bct, bcd, g,
-                                     make_double4(Gb[0], Gb[1], Gb[2], Gb[3]));
-    Uib[0] += r.x; Uib[1] += r.y; Uib[2] += r.z; Uib[3] += r.w;
+template <bool CALL>
+__device__ __forceinline__ void ghost_vjp_of(const double* Ui, double nx, double ny, int bct, const double* bcd,
+                                             double g, const double* Gb, double* Uib) {
+    if constexpr (CALL) {
+        const double4 r = ghost_vjp_call(make_double4(Ui[0], Ui[1], Ui[2], Ui[3]), nx, ny, bct, bcd, g,
+                                         make_double4(Gb[0], Gb[1], Gb[2], Gb[3]));
+        Uib[0] += r.x; Uib[1] += r.y; Uib[2] += r.z; Uib[3] += r.w;
+    } else {
+        ghost_vjp(Ui, nx, ny, bct, bcd, g, Gb, Uib);
+    }
 }
 
 }  // namespace adj
