@@ -246,19 +246,23 @@ k_phys_stage(const StageArgsT<T> a) {
 
     // ---- A: loads; transformed fluxes into shared memory; common fluxes
     constexpr bool kRef = UsesRef<T>::value;
-    // (loads first, the edge record ahead of all: the neighbour's row hangs on it)
+    // (loads first, the edge record ahead of all, as the neighbour's row hangs on
+    // it; in FP32 the reference state before it from P2 up: at P3, where every
+    // thread holds both points, a step takes 1032 instead of 1116 us on
+    // 320 x 317 and 60.6 instead of 64.7 on 12 x 9 (Roe); at P1 64.7 instead of 60.3)
     T u[4], Jd = T(1);
     T Fd[4] = {T(0), T(0), T(0), T(0)};
     T ue[4] = {T(0), T(0), T(0), T(0)};   // reference state (mixed form)
     T nr[3], qo[4], qn[4], ji[4];
     double ud[4];
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
+    if (kRef && P > 1 && valid) load_state(a.U + e * NSP * 4, ue);
     if (is_fp) {
         r = a.edges[e * 4 + edge];
         load4_now(a.Tin + (e * NFT + kf) * 4, qo);
         load_normal(normal_rec<N1>(a, e, edge, fp), nr);
     }
-    if (kRef && valid) load_state(a.U + e * NSP * 4, ue);
+    if (kRef && P == 1 && valid) load_state(a.U + e * NSP * 4, ue);
     if (is_sp) {
         const long long idx = e * NSP + ks;
         stage_state(a, idx, ud, u);
