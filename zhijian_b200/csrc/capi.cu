@@ -61,7 +61,7 @@ struct zj_solver {
     bool mixed = false;
     int nrm_pp = 0;             // curved elements in physics mode: normals per flux point
     float* fT[3] = {nullptr, nullptr, nullptr};
-    float* fTQ = nullptr;
+    float* fTQ = nullptr;       // viscous shares of the faces
     float* fJinv = nullptr;
     float* fJ = nullptr;
     float* fOps = nullptr;
@@ -605,10 +605,11 @@ zj_status create_impl(const zj_mesh_desc* mesh, const zj_params* params, const i
     }
     if (!s->mixed) {
         for (int i = 0; i < 3; ++i) { ZJ_ALLOC(s->dT[i], s->trace_n); }
+        // (gradient traces, which the adjoint reads, are twice the shares' size)
         if (is_ns(s)) { ZJ_ALLOC(s->dTQ, 2 * s->trace_n); }
     } else {
         for (int i = 0; i < 3; ++i) { ZJ_ALLOC(s->fT[i], s->trace_n); }
-        if (is_ns(s)) { ZJ_ALLOC(s->fTQ, 2 * s->trace_n); }
+        if (is_ns(s)) { ZJ_ALLOC(s->fTQ, s->trace_n); }
         ZJ_ALLOC(s->fJinv, Jinv.size());
         ZJ_ALLOC(s->fJ, J.size());
         ZJ_ALLOC(s->fOps, packed.size());
@@ -689,8 +690,8 @@ zj_status create_impl(const zj_mesh_desc* mesh, const zj_params* params, const i
         const size_t tsz = s->mixed ? sizeof(float) : sizeof(double);
         e = dalloc(&s->dSendRows, ni);
         if (e == cudaSuccess) e = dalloc(&s->dRecvRows, ni);
-        if (e == cudaSuccess) e = cudaMalloc(&s->dSendBuf, std::max<size_t>(ni, 1) * s->n1 * 8 * tsz);
-        if (e == cudaSuccess) e = cudaMalloc(&s->dRecvBuf, std::max<size_t>(ni, 1) * s->n1 * 8 * tsz);
+        if (e == cudaSuccess) e = cudaMalloc(&s->dSendBuf, std::max<size_t>(ni, 1) * s->n1 * 4 * tsz);
+        if (e == cudaSuccess) e = cudaMalloc(&s->dRecvBuf, std::max<size_t>(ni, 1) * s->n1 * 4 * tsz);
         if (e == cudaSuccess && ni)
             e = cudaMemcpy(s->dSendRows, send.data(), ni * 4, cudaMemcpyHostToDevice);
         if (e == cudaSuccess && ni)
@@ -1042,7 +1043,7 @@ zj_status ensure_diff(zj_solver* s) {
     ZJ_ALLOC(s->xBC, s->n_bcd);
     ZJ_ALLOC(s->xNrm, s->n_nrm);
     ZJ_ALLOC(s->xT, s->trace_n);
-    ZJ_ALLOC(s->xTQ, 2 * s->trace_n);
+    if (is_ns(s)) { ZJ_ALLOC(s->xTQ, s->trace_n); }
     ZJ_ALLOC(s->xPart, (size_t)dual_grid(s->P, s->E));
     const size_t fpn = (size_t)s->E * 4 * s->n1 * 4;
     ZJ_ALLOC(s->aDb, fpn);
