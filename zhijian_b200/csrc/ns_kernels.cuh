@@ -48,14 +48,8 @@
 #ifndef ZJ_NS_MIN_BLOCKS
 #define ZJ_NS_MIN_BLOCKS 4        // FP64 stage kernel (128 registers)
 #endif
-#ifndef ZJ_NSG_MIN_BLOCKS
-#define ZJ_NSG_MIN_BLOCKS 8       // FP64 point-per-thread gradient kernel
-#endif
 #ifndef ZJ_NS32_MIN_BLOCKS
 #define ZJ_NS32_MIN_BLOCKS 8      // mixed-precision stage kernel (64 registers)
-#endif
-#ifndef ZJ_NSG32_MIN_BLOCKS
-#define ZJ_NSG32_MIN_BLOCKS 12    // mixed-precision point-per-thread gradient kernel
 #endif
 // Threads per CTA of the gradient kernel by lines (rounded down to whole
 // elements): 64 spread a coarse mesh over more SMs and interleave more phases;
@@ -65,13 +59,13 @@
 #define ZJ_LINE_THREADS 64
 #endif
 #ifndef ZJ_NSL_MIN_BLOCKS
-#define ZJ_NSL_MIN_BLOCKS 4       // FP64 gradient kernel by lines (128 registers)
+#define ZJ_NSL_MIN_BLOCKS 4       // FP64 gradient kernel by lines (128 registers; 24 B of spills at P5)
 #endif
 #ifndef ZJ_NSL32_MIN_BLOCKS
-#define ZJ_NSL32_MIN_BLOCKS 8     // mixed-precision gradient kernel by lines (64 registers)
+#define ZJ_NSL32_MIN_BLOCKS 8     // mixed-precision gradient kernel by lines (64 registers; 4 B of spills at P3)
 #endif
 #ifndef ZJ_NSL32_MIN_BLOCKS_HI
-#define ZJ_NSL32_MIN_BLOCKS_HI 6  // the same from P4 up (no spills)
+#define ZJ_NSL32_MIN_BLOCKS_HI 6  // the same from P4 up (80 registers; 28 B of spills at P5)
 #endif
 
 namespace zj {
@@ -84,13 +78,11 @@ template <typename T, int P> struct NSMinBlocks;
 constexpr int per_cta(int blocks128) { return blocks128 * 128 / kCtaThreads > 0 ? blocks128 * 128 / kCtaThreads : 1; }
 template <int P> struct NSMinBlocks<double, P> {
     static constexpr int stage = per_cta(ZJ_NS_MIN_BLOCKS);
-    static constexpr int grad = per_cta(ZJ_NSG_MIN_BLOCKS);
 };
 template <int P> struct NSMinBlocks<float, P> {
     static constexpr int stage = per_cta(ZJ_NS32_MIN_BLOCKS);
-    static constexpr int grad = per_cta(ZJ_NSG32_MIN_BLOCKS);
 };
-template <int P> struct NSMinBlocks<Dual, P> { static constexpr int stage = 1, grad = 1; };
+template <int P> struct NSMinBlocks<Dual, P> { static constexpr int stage = 1; };
 
 // Corrected gradient at solution point (i, j) of one element: su is the
 // element's state tile, du its face jumps U_c - U_own in the flux-point tile.
@@ -161,8 +153,9 @@ __device__ __forceinline__ void viscous_share(const StageArgsT<T>& a, const Edge
     boundary_viscous_closure(r, a.bc, nx, ny, f);
 }
 
+// Gradient of the dual-number instantiation, a thread per point.
 template <int P, typename T>
-__global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS, NSMinBlocks<T, P>::grad)
+__global__ void __launch_bounds__(Shape<P, EbDiv<T>::value>::THREADS)
 k_ns_grad(const StageArgsT<T> a) {
     using S = Shape<P, EbDiv<T>::value>;
     constexpr int N1 = S::N1, NSP = S::NSP, NFT = S::NFT, TPE = S::TPE, EB = S::EB;
@@ -187,22 +180,12 @@ k_ns_grad(const StageArgsT<T> a) {
     int i, j;
     lane_point<N1>(k, i, j);
 
-    constexpr bool kRef = UsesRef<T>::value;
     T ji[4];
     if (is_sp) {
         const long long idx = e * NSP + j * N1 + i;
         T u[4];
-        if constexpr (kRef) {
-            // D (U - U_e): the reference drops out of the derivative exactly
-            double ud[4];
-            T ue[4];
-            gload4(a.U + idx * 4, ud);
-            load_state(a.U + e * NSP * 4, ue);
-            state_minus_ref(ud, ue, u);
-        } else {
-            double ud[4];
-            stage_state(a, idx, ud, u);
-        }
+        double ud[4];
+        stage_state(a, idx, ud, u);
         load4_nc(a.Jinv + idx * 4, ji);
         store4(sU + el * FP + j * RP + 4 * i, u);
     }
@@ -228,14 +211,11 @@ k_ns_grad(const StageArgsT<T> a) {
         T t[8];
         state_trace<P>(sQx + el * FP, sOps, fl, t);
         state_trace<P>(sQy + el * FP, sOps, fl, t + 4);
-        if (a.GQ) gstore8(a.GQ + (e * NFT + kf) * 8, t);
-        if (a.FVout) {
-            T Ua[4], fv[4];
+        T Ua[4], fv[4];
 #pragma unroll
-            for (int v = 0; v < 4; ++v) Ua[v] = T(0.5) * (f.qo[v] + f.qn[v]);
-            viscous_share(a, f.r, f.nx, f.ny, Ua, t, fv);
-            gstore4(a.FVout + (e * NFT + kf) * 4, fv);
-        }
+        for (int v = 0; v < 4; ++v) Ua[v] = T(0.5) * (f.qo[v] + f.qn[v]);
+        viscous_share(a, f.r, f.nx, f.ny, Ua, t, fv);
+        gstore4(a.FVout + (e * NFT + kf) * 4, fv);
     }
 }
 
@@ -440,11 +420,13 @@ k_ns_grad_lines(const StageArgsT<T> a) {
             tB[4 + v] = fma_any(wb, Qy, tB[4 + v]);
         }
     }
-    if (a.GQ) {
-        gstore8(a.GQ + (e * NFT + eA * N1 + fA) * 8, tA);
-        gstore8(a.GQ + (e * NFT + eB * N1 + fB) * 8, tB);
+    if constexpr (sizeof(T) == 8) {   // the adjoint's gradient traces (FP64 only), with the shares or alone
+        if (a.GQ) {
+            gstore8(a.GQ + (e * NFT + eA * N1 + fA) * 8, tA);
+            gstore8(a.GQ + (e * NFT + eB * N1 + fB) * 8, tB);
+        }
+        if (!a.FVout) return;
     }
-    if (!a.FVout) return;
 #pragma unroll
     for (int s2 = 0; s2 < 2; ++s2) {
         const int ed = s2 ? eB : eA, fp = s2 ? fB : fA;

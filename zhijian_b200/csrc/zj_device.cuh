@@ -151,14 +151,8 @@ __device__ __forceinline__ void load4_now(const float* p, float* v) {
 __device__ __forceinline__ void store4(float* p, const float* v) {
     *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
 }
-// Global float rows: four values are one 16-byte access; eight (a gradient
-// trace point, 32-byte aligned like the double rows) one 32-byte access.
+// Global float rows: four values are one 16-byte access.
 __device__ __forceinline__ void gstore4(float* p, const float* v) { store4(p, v); }
-__device__ __forceinline__ void gstore8(float* p, const float* v) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]),
-                 "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                 : "memory");
-}
 
 __device__ __forceinline__ double ldg_any(const double* p) { return __ldg(p); }
 __device__ __forceinline__ float ldg_any(const float* p) { return __ldg(p); }
@@ -377,11 +371,6 @@ __device__ __forceinline__ V4<T> v4_load(const T* p) {
 __device__ __forceinline__ V4<float> v4_load(const float* p) {
     const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(p);
     return {t.x, t.y};
-}
-template <typename T>
-__device__ __forceinline__ void v4_store(T* p, const V4<T>& a) { store4(p, a.v); }
-__device__ __forceinline__ void v4_store(float* p, const V4<float>& a) {
-    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(a.a, a.b);
 }
 
 // Weights of an operator row in shared memory.
