@@ -250,14 +250,14 @@ k_adj_euler(const AdjArgs a) {
 }
 
 // ---------------------------------------------------- pass B, Navier-Stokes --
-// Up to P3 4 CTAs of 60 to 64 threads per SM (about 250 registers, no spills) with
-// the ghost state's transpose as a call; from P4 up 6 CTAs (168 registers,
-// spills of 0.3 to 0.4 KB) with the transpose inlined, as these CTAs' 50 or 36
-// threads leave their warps partly empty. Transposed residual, the first form
-// against the second: P3 HLLC 50 and 57 us on 40 x 37, P1 Rusanov 62 and 70 on
-// 90 x 87; P4 HLLC 79 and 69 on 40 x 37, P5 Roe 455 and 416 on 160 x 157.
-template <int P> constexpr bool kGhostCall = P <= 3;
-template <int P> constexpr int kAdjNsBlocks = P <= 3 ? 4 : 6;
+// Up to P4 4 CTAs of 50 to 64 threads per SM (about 250 registers, no spills) with
+// the ghost state's transpose as a call; at P5, whose CTAs' 36 threads leave a
+// warp almost empty, 6 CTAs (168 registers, spills of 0.4 KB) with the
+// transpose inlined. Transposed residual, the first form against the second: P3 HLLC
+// 50 and 57 us on 40 x 37, P4 Rusanov 179 and 183 on 90 x 87 (HLLC on 40 x 37, just
+// over a wave at 4 CTAs, 79 and 69), P5 Roe 455 and 416 on 160 x 157.
+template <int P> constexpr bool kGhostCall = P <= 4;
+template <int P> constexpr int kAdjNsBlocks = P <= 4 ? 4 : 6;
 
 template <int P, int RIEM>
 __global__ void __launch_bounds__(Shape<P, 2>::THREADS, kAdjNsBlocks<P>)
