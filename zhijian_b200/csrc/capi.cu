@@ -1270,7 +1270,14 @@ zj_status zj_adjoint_run(zj_solver* s, double dt, int nsteps, int k_ckpt, double
     if (misaligned(G_dev)) return fail(s, ZJ_ERR_ARG, kAlignMsg);
     if (nsteps < 1 || k_ckpt < 1 || !std::isfinite(dt)) return fail(s, ZJ_ERR_ARG, "bad dt, nsteps or k_ckpt");
     zj_status st = diff_supported(s);
-    if (st == ZJ_OK) st = ensure_diff(s);
+    if (st != ZJ_OK) return st;
+    // refused before anything is queued: the wait at the end would end the
+    // capture with an error, and the kept block could not be freed in it
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    ZJ_CK(s, cudaStreamIsCapturing(s->stream, &cs), "capture query");
+    if (cs != cudaStreamCaptureStatusNone)
+        return fail(s, ZJ_ERR_CUDA, "zj_adjoint_run waits for its stream and cannot run under stream capture");
+    st = ensure_diff(s);
     if (st == ZJ_OK) st = set_dt(s, dt);
     if (st != ZJ_OK) return st;
     const int n_ck = (nsteps + k_ckpt - 1) / k_ckpt;
