@@ -457,6 +457,12 @@ cudaError_t tri_traces_t(const StageArgsT<T>& a, const int32_t* elist, long long
     return cudaGetLastError();
 }
 
+// Triangles ask for the quads' split, also where their own kernels would want more
+// for the CTAs of their launch bounds (inviscid, per SM: FP64 P5 121 KB against 93,
+// FP32 P4 104 against 86 and P5 128 against 72). Six inviscid steps of the shear
+// layer, this split against one that fits the triangles (Roe): FP32 P5 275 and 368 us
+// at 60 x 57, 4222 and 4045 at 320 x 317; FP32 P4 296 and 399, 3037 and 3029; FP64 P5
+// 413 and 450, 7185 and 6868: what large meshes would gain the others lose five times over.
 template <int P, typename T>
 cudaError_t tri_grad_t(const StageArgsT<T>& a, const int32_t* elist, long long n, cudaStream_t s) {
     using S = TriShape<P, T>;

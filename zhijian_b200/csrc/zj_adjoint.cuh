@@ -3,7 +3,7 @@
 //   euler_flux_vjp   (dF/dU)^T Fbar + (dG/dU)^T Gbar, closed form
 //   viscous_vjp      transposed viscous flux w.r.t. the state and the
 //                    conservative gradients, closed form (reverse sweep of
-//                    phys::viscous_flux)
+//                    phys::viscous_flux_f)
 //   riemann_vjp      transposed common flux w.r.t. both states: the Roe
 //                    solver by its reverse sweep (roe_vjp), Rusanov and HLLC
 //                    column by column from tangent evaluations on dual
@@ -54,7 +54,7 @@ __device__ __forceinline__ void euler_flux_vjp(const double* s, double g, const 
     ub[0] += rb; ub[1] += mb; ub[2] += nb; ub[3] += Eb;
 }
 
-// Reverse sweep of phys::viscous_flux: given Fvb, Gvb (components 1..3; the
+// Reverse sweep of phys::viscous_flux_f: given Fvb, Gvb (components 1..3; the
 // mass components of the viscous flux are zero), adds the adjoints of the
 // state s and of the gradients dx = dU/dx, dy = dU/dy into sb, dxb, dyb.
 // Returns Fvb . Fv + Gvb . Gv: the viscous flux is proportional to 1/Re, so
@@ -63,7 +63,8 @@ __device__ __forceinline__ double viscous_vjp(const double* s, const double* dx,
                                             double g, double Re, double Pr, const double* Fvb,
                                             const double* Gvb, double* sb, double* dxb,
                                             double* dyb) {
-    // forward recomputation (the operations of phys::viscous_flux)
+    // forward recomputation (phys::viscous_flux_f, with mu and the conductivity's
+    // factor by division)
     const double ir = rcp_any(s[0]);
     const double u = s[1] * ir, v = s[2] * ir;
     const double dudx = (dx[1] - u * dx[0]) * ir, dudy = (dy[1] - u * dy[0]) * ir;

@@ -441,9 +441,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // Split of an SM's 256 KB between shared memory and L1.  Kernels that follow one
 // another in a step ask for the same split (another one would have to wait for
-// the SM to drain): as much shared memory as the one with the larger demand
-// needs at full occupancy, per CTA its own and the 1 KB the system takes, the
-// rest L1.  The L1 serves the second reads of states, edge records and
+// the SM to drain): as much shared memory as the quad kernel with the larger
+// demand needs for the CTAs its launch bound makes resident, per CTA its own and
+// the 1 KB the system takes, the rest L1 (triangles follow the quads, whatever
+// they need themselves: tri_kernels.cuh; dual numbers take all).  The L1 serves the second reads of states, edge records and
 // neighbours' rows; against the largest shared-memory split (256 x 256, P3, per
 // step): FP32 222 -> 212 us, FP64 373 -> 364 us, compat 169 -> 166 us; curved
 // P4 Euler FP64 116 -> 108 us.

@@ -32,7 +32,7 @@ constexpr int32_t kEdgeRight = 1;    // this element is the face's right side
 constexpr int32_t kEdgeBoundary = 2; // boundary face (ghost state)
 constexpr int32_t kEdgeOrphan = 4;   // edge on no face (non-manifold): no correction
 // A face cut by a mesh partition (with kEdgeBoundary: its neighbour's trace
-// and gradient trace sit in a ghost row, filled by the halo exchange instead
+// and viscous share sit in a ghost row, filled by the halo exchange instead
 // of a boundary condition; kEdgeRight as on an interior face).
 constexpr int32_t kEdgeInterface = 8;
 ZJ_HD inline int32_t edge_bc_type(int32_t flags) { return (flags >> 8) & 0xF; }

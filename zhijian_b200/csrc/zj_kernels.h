@@ -76,7 +76,8 @@ cudaError_t launch_phys_stage(int P, int riemann, const StageArgs32& a, cudaStre
 // Physics-mode traces of a.U into a.Tout, boundary ghost rows included.
 cudaError_t launch_phys_traces(int P, const StageArgs& a, cudaStream_t s);
 cudaError_t launch_phys_traces(int P, const StageArgs32& a, cudaStream_t s);
-// Navier-Stokes: gradient traces of a stage state, then the stage itself.
+// Navier-Stokes: viscous shares of a stage state's faces (and gradient traces where
+// a.GQ asks for them), then the stage itself.
 cudaError_t launch_ns_grad(int P, const StageArgs& a, cudaStream_t s);
 cudaError_t launch_ns_grad(int P, const StageArgs32& a, cudaStream_t s);
 cudaError_t launch_ns_stage(int P, int riemann, const StageArgs& a, cudaStream_t s);
@@ -89,7 +90,7 @@ cudaError_t launch_ns_grad(int P, const StageArgsDual& a, cudaStream_t s);
 cudaError_t launch_ns_stage(int P, int riemann, const StageArgsDual& a, cudaStream_t s);
 int dual_grid(int P, long long n_elem);
 // Triangles (tri_kernels.cuh): what = 0 traces (+ ghost rows) of a.U into
-// a.Tout, 1 gradient traces (Navier-Stokes), 2 residual / stage; over the
+// a.Tout, 1 viscous shares (Navier-Stokes), 2 residual / stage; over the
 // triangle list elist[0..n).  a.ops holds the packed triangle operators.
 cudaError_t launch_tri(int what, int P, int riemann, bool viscous, const StageArgs& a, const int32_t* elist,
                        long long n, cudaStream_t s);
