@@ -248,8 +248,9 @@ k_phys_stage(const StageArgsT<T> a) {
     constexpr bool kRef = UsesRef<T>::value;
     // (loads first, the edge record ahead of all, as the neighbour's row hangs on
     // it; in FP32 the reference state before it from P2 up: at P3, where every
-    // thread holds both points, a step takes 1032 instead of 1116 us on
-    // 320 x 317 and 60.6 instead of 64.7 on 12 x 9 (Roe); at P1 64.7 instead of 60.3)
+    // thread holds both points, six steps take 1024 instead of 1105 us on
+    // 320 x 317 and 62.6 instead of 64.7 on 12 x 9 (Roe), but only with the
+    // traces' pointer taken behind that load; at P1 64.7 instead of 60.3)
     T u[4], Jd = T(1);
     T Fd[4] = {T(0), T(0), T(0), T(0)};
     T ue[4] = {T(0), T(0), T(0), T(0)};   // reference state (mixed form)
@@ -257,9 +258,10 @@ k_phys_stage(const StageArgsT<T> a) {
     double ud[4];
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
     if (kRef && P > 1 && valid) load_state(a.U + e * NSP * 4, ue);
+    const T* Tin = after_wait(a.Tin);
     if (is_fp) {
         r = a.edges[e * 4 + edge];
-        load4_now(a.Tin + (e * NFT + kf) * 4, qo);
+        load4_now(Tin + (e * NFT + kf) * 4, qo);
         load_normal(normal_rec<N1>(a, e, edge, fp), nr);
     }
     if (kRef && P == 1 && valid) load_state(a.U + e * NSP * 4, ue);
@@ -272,7 +274,7 @@ k_phys_stage(const StageArgsT<T> a) {
     }
     const bool face = is_fp && !(r.flags & kEdgeOrphan);
     const bool bc_face = is_fp && boundary_condition_edge(r);
-    if (face) load4_now(a.Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
+    if (face) load4_now(Tin + (neighbour_row(r, a.n_elem) * N1 + (N1 - 1 - fp)) * 4, qn);
     if (is_sp) {
         T F[4], G[4];
         euler_flux(u, g, F, G);
