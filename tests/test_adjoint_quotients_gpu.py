@@ -29,7 +29,7 @@ __global__ void k(const double* T, double Re, double* pw, double* mu, double* eb
     const double s[4] = {1.0, 0.0, 0.0, T[i]}, dx[4] = {0.0, 0.0, 0.0, 0.0}, dy[4] = {0.0, 1.0, 0.0, 0.0};
     const double Fb[4] = {0.0, 0.0, 1.0, 0.0}, Gb[4] = {0.0, 0.0, 0.0, 0.0};
     double sb[4] = {0.0, 0.0, 0.0, 0.0}, xb[4] = {0.0, 0.0, 0.0, 0.0}, yb[4] = {0.0, 0.0, 0.0, 0.0};
-    mu[i] = zj::adj::viscous_vjp(s, dx, dy, 2.0, Re, 0.72, Fb, Gb, sb, xb, yb);
+    mu[i] = zj::adj::viscous_vjp(s, dx, dy, 2.0, Re, 2.0 / 0.72, Fb, Gb, sb, xb, yb);
     eb[i] = sb[3];
     pw[i] = zj::zj_pow07(T[i]);
 }

@@ -283,7 +283,7 @@ k_adj_ns(const AdjArgs a) {
     const bool is_sp = valid && k < NSP, is_fp = valid && k < NFT;
     const int edge = k / N1, fp = k - edge * N1;
     const int i = k % N1, j = k / N1;
-    const double g = a.gamma, Re = a.Re, Pr = a.Pr;
+    const double g = a.gamma, Re = a.Re, kfac = a.kfac;
 
     // ---- 1: loads
     EdgeRec r{-1, 0, kEdgeOrphan, 0};
@@ -331,7 +331,7 @@ k_adj_ns(const AdjArgs a) {
     __syncthreads();
 
     // ---- 2: transposed fluxes at the solution points; face adjoints
-    double re_acc = 0.0;     // L . dR/dRe of this thread's viscous fluxes
+    double re_acc = 0.0;     // Re L . dR/dRe of this thread's viscous fluxes
     double ub[4] = {0.0, 0.0, 0.0, 0.0}, Qxb[4] = {0.0, 0.0, 0.0, 0.0}, Qyb[4] = {0.0, 0.0, 0.0, 0.0};
     if (is_sp) {
         double Qx[4], Qy[4];
@@ -346,7 +346,7 @@ k_adj_ns(const AdjArgs a) {
             mGb[v] = -Gb[v];
         }
         adj::euler_flux_vjp(u, g, Fb, Gb, ub);
-        re_acc -= adj::viscous_vjp(u, Qx, Qy, g, Re, Pr, mFb, mGb, ub, Qxb, Qyb) / Re;
+        re_acc -= adj::viscous_vjp(u, Qx, Qy, g, Re, kfac, mFb, mGb, ub, Qxb, Qyb);
     }
     double tb[4] = {0.0, 0.0, 0.0, 0.0};
     if (is_fp) {
@@ -377,8 +377,8 @@ k_adj_ns(const AdjArgs a) {
                 Fvb[v] = -Fnb[v] * nx;
                 Gvb[v] = -Fnb[v] * ny;
             }
-            const double dv = adj::viscous_vjp(Ua, dxa, dya, g, Re, Pr, Fvb, Gvb, Uab, dxb, dyb);
-            if (!right) re_acc -= dv / Re;   // once per face: on its left element
+            const double dv = adj::viscous_vjp(Ua, dxa, dya, g, Re, kfac, Fvb, Gvb, Uab, dxb, dyb);
+            if (!right) re_acc -= dv;   // once per face: on its left element
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 ULb[v] += 0.5 * Uab[v];
@@ -397,7 +397,7 @@ k_adj_ns(const AdjArgs a) {
         store4(sTQ + el * 2 * DS + k * 8 + 4, tq + 4);
     }
     if (a.re_part) {
-        const double bs = block_sum(re_acc, sRed);
+        const double bs = block_sum(re_acc / Re, sRed);
         if (tid == 0) a.re_part[blockIdx.x] = bs;
     }
     __syncthreads();   // sA, sU, sD free from here

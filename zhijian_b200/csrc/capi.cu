@@ -1119,7 +1119,7 @@ zj_status vjp_core(zj_solver* s, const double* U, const double* L, double* W, do
     g.U = U; g.L = L; g.W = W; g.T = T; g.TQ = TQ;
     g.Db = s->aDb; g.Tb = s->aTb; g.DUb = s->aDUb;
     g.Jinv = s->dJinv; g.J = s->dJ; g.edges = s->dEdges; g.enrm = s->dNrm; g.bc = s->dBC; g.ops = s->dOps;
-    g.n_elem = s->E; g.gamma = s->prm.gamma; g.Re = s->prm.Re; g.Pr = s->prm.Pr;
+    g.n_elem = s->E; g.gamma = s->prm.gamma; g.Re = s->prm.Re; g.kfac = g.gamma / ((g.gamma - 1.0) * s->prm.Pr);
     const bool re = is_ns(s) && re_weight != 0.0;
     g.re_part = re ? s->aRePart : nullptr;
     g.out = o.out; g.X0 = o.X0; g.X1 = o.X1; g.X2 = o.X2;

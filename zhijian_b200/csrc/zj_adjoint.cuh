@@ -57,14 +57,14 @@ __device__ __forceinline__ void euler_flux_vjp(const double* s, double g, const 
 // Reverse sweep of phys::viscous_flux_f: given Fvb, Gvb (components 1..3; the
 // mass components of the viscous flux are zero), adds the adjoints of the
 // state s and of the gradients dx = dU/dx, dy = dU/dy into sb, dxb, dyb.
-// Returns Fvb . Fv + Gvb . Gv: the viscous flux is proportional to 1/Re, so
-// minus this over Re is the flux adjoint's Reynolds-number derivative.
+// kfac = gamma/((gamma-1) Pr).  Returns Fvb . Fv + Gvb . Gv: the viscous flux is
+// proportional to 1/Re, so minus this over Re is the flux adjoint's
+// Reynolds-number derivative.
 __device__ __forceinline__ double viscous_vjp(const double* s, const double* dx, const double* dy,
-                                            double g, double Re, double Pr, const double* Fvb,
+                                            double g, double Re, double kfac, const double* Fvb,
                                             const double* Gvb, double* sb, double* dxb,
                                             double* dyb) {
-    // forward recomputation (phys::viscous_flux_f, with mu and the conductivity's
-    // factor by division)
+    // forward recomputation (phys::viscous_flux_f, with mu by division)
     const double ir = rcp_any(s[0]);
     const double u = s[1] * ir, v = s[2] * ir;
     const double dudx = (dx[1] - u * dx[0]) * ir, dudy = (dy[1] - u * dy[0]) * ir;
@@ -77,7 +77,7 @@ __device__ __forceinline__ double viscous_vjp(const double* s, const double* dx,
     const double dpdy = c * (dy[3] - 0.5 * dy[0] * q2 - s[0] * (u * dudy + v * dvdy));
     const double dTdx = (dpdx - Tm * dx[0]) * ir, dTdy = (dpdy - Tm * dy[0]) * ir;
     const double mu = zj_pow07(Tm) / Re;
-    const double kc = g / (c * Pr);
+    const double kc = kfac;
     const double k = mu * kc;
     const double div = dudx + dvdy, lam = (-2.0 / 3.0) * mu;
     const double txx = 2.0 * mu * dudx + lam * div, tyy = 2.0 * mu * dvdy + lam * div;

@@ -137,7 +137,8 @@ struct AdjArgs {
     const double* bc;
     const double* ops;
     long long n_elem;
-    double gamma, Re, Pr;
+    double gamma, Re;
+    double kfac;            // gamma/((gamma-1) Pr), the conductivity's factor
     double* re_part;        // optional, Navier-Stokes: per-CTA L . dR/dRe, adj_ns_grid entries
     // optional fused output: out = c0 X0 + c1 X1 + c2 X2 + cw (dR/dU)^T L
     // (an SSP-RK3 stage's adjoint update; X* may be NULL when c* is 0, out may
